@@ -3,14 +3,18 @@
 // A CTA of 4 warps computes an 8 TM x 8 TN WN complex tile: WN warps side by side along N, each with TM x TN
 // tiles of 8 x 8, and WK = 4 / WN groups of them that split the K steps and are summed at the end.  A step of 4
 // along K is four mma.sync m8n8k4 per 8 x 8 tile (Re C += Re A Re B - Im A Im B, Im C += Re A Im B + Im A Re B),
-// ordered so that two products into the same accumulator lie TN..2 TN instructions apart (back to back they
+// ordered so that two products into the same accumulator lie 2 TM TN instructions apart (back to back they
 // wait for one another's latency).  Operands stay interleaved complex in shared memory: 16-byte cp.async
 // straight from the index-mapped global element into a ring of STAGES K blocks, zero fill outside the matrix,
 // one barrier per block.  K-fastest operands are kept [row][k] with 4 spare elements a row, the others [k][row]
 // with 2 spare, so that the 8 lanes of a 128-bit fragment read hit different banks in both.
 //
 // Two CTAs of 128 threads share an SM (up to 255 registers a thread): one of them stores its tile or fills its
-// ring while the other multiplies.  What bounds it is the FP64 tensor pipe (37 TFLOP/s from registers).
+// ring while the other multiplies.  What bounds it is the FP64 tensor pipe (37 TFLOP/s from registers): 71 % of it
+// on 150 x 150 x 10816, half on contractions as short as K = 26, where the index maps and the stores count.  Copies
+// issued between the products instead of before them were slower (their address loads stall the warp that multiplies).
+// Exchange of a Fock build at nk = 27, nao = 40, NQ = 250: 29.4 -> 10.0 ms against the 64 x 64 kernel with register
+// staging that this one replaced.
 // Contractions with few tiles split K over a cluster of up to 8 CTAs and sum the parts through distributed
 // shared memory in rank order, so a result never depends on timing.
 #include <cooperative_groups.h>
@@ -171,26 +175,36 @@ __global__ void __launch_bounds__(NT, 2)
       for (int kq = 0; kq < BK / 4 / T::WK; ++kq) {
         const int k4 = kq * T::WK + wk;
         if (k4 >= ksteps) break;
-        double bre[TN], bim[TN];
+        double are[TM], aim[TM], bre[TN], bim[TN], nim[TN];
 #pragma unroll
         for (int j = 0; j < TN; ++j) {
           const cplx v = sb[j * 8 * brs + k4 * 4 * bks];
           bre[j] = v.x;
           bim[j] = flip(v.y, sgb);
+          nim[j] = flip(v.y, sgb ^ 0x80000000u);
         }
 #pragma unroll
         for (int i = 0; i < TM; ++i) {
           const cplx v = sa[i * 8 * ars + k4 * 4 * aks];
-          const double are = v.x, aim = flip(v.y, sga), nim = flip(v.y, sga ^ 0x80000000u);
-#pragma unroll
-          for (int j = 0; j < TN; ++j) dmma(cr[i][j], are, bre[j]);
-#pragma unroll
-          for (int j = 0; j < TN; ++j) dmma(ci[i][j], are, bim[j]);
-#pragma unroll
-          for (int j = 0; j < TN; ++j) dmma(cr[i][j], nim, bim[j]);
-#pragma unroll
-          for (int j = 0; j < TN; ++j) dmma(ci[i][j], aim, bre[j]);
+          are[i] = v.x;
+          aim[i] = flip(v.y, sga);
         }
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) dmma(cr[i][j], are[i], bre[j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) dmma(ci[i][j], are[i], bim[j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) dmma(cr[i][j], aim[i], nim[j]);
+#pragma unroll
+        for (int i = 0; i < TM; ++i)
+#pragma unroll
+          for (int j = 0; j < TN; ++j) dmma(ci[i][j], aim[i], bre[j]);
       }
     }
     cp_wait<0>();
