@@ -57,7 +57,7 @@ enum ScratchSlot {
   SL_IO_S1, SL_IO_H, SL_DM, SL_PINV, SL_SPLIT0, SL_HF_TAB, SL_X2C_DM, SL_X2C_S, SL_X2C_F, SL_X2C_GAB, SL_X2C_GBA,
   SL_X2C_SIG, SL_Q0_Y, SL_Q0_T, SL_Q0_D, SL_Q0_E, SL_Q0_S, SL_ADJ_TH, SL_ADJ_PTW, SL_ADJ_W, SL_ADJ_WB,
   SL_ADJ_PTWB, SL_ADJ_PWB, SL_ADJ_THB, SL_ADJ_XB, SL_ADJ_AB, SL_ADJ_P0B, SL_ADJ_P0HB, SL_ADJ_X3, SL_ADJ_TAB, SL_ADJ_TQ, SL_ADJ_VBF, SL_ADJ_VBH,
-  SL_SINK, SL_COUNT
+  SL_SINK, SL_INV_BAD, SL_DY_TR, SL_COUNT
 };
 
 struct SplitEngine;
@@ -175,8 +175,15 @@ void energy(Context& c, const cplx* G, const cplx* Sigma1, const cplx* Sigma_tau
 // linear algebra helpers (linalg.cu)
 void hermitize_batched(cplx* X, int64_t nmat, int n, double scale, cudaStream_t st);
 void invert_small_batched(const cplx* A, cplx* Ainv, int64_t nmat, int n, cudaStream_t st);
-void invert_large_batched(const cplx* A, cplx* Ainv, cplx* aug, int64_t nmat, int n, bool herm_from_lower,
-                          bool identity_minus, cudaStream_t st);
+// G[w][sk] = (z_w S[sk] - X[w][sk])^-1 with z_w = mu + i wn[w], and tr[w][sk] = Tr(G[w][sk] S[sk])
+void invert_dyson_batched(const cplx* X, const cplx* S, const double* wn, double mu, cplx* G, int64_t nw, int64_t nsk,
+                          int n, cudaStream_t st);
+void trace_dyson_batched(const cplx* X, const cplx* S, const double* wn, double mu, cplx* tr, int64_t nw, int64_t nsk,
+                         int n, cudaStream_t st);
+// Inverse of the Hermitian matrix that the lower triangle and real diagonal of A (or I - A) define; `aug` holds
+// nmat * 2 n^2 elements, `bad` nmat flags.  The result is Hermitian.
+void invert_large_batched(const cplx* A, cplx* Ainv, cplx* aug, int* bad, int64_t nmat, int n, bool identity_minus,
+                          cudaStream_t st);
 void scale_inplace(cplx* X, int64_t count, double s, cudaStream_t st);
 
 }  // namespace gb200

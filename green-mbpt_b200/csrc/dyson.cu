@@ -38,47 +38,45 @@ __global__ void build_x_kernel(const cplx* H, const cplx* S1, const cplx* Sw, cp
   }
 }
 
-// A[n][s][k] = (i w_n + mu) S - X[n][s][k]
-__global__ void build_a_kernel(const cplx* S, const cplx* X, const double* wn, double mu, cplx* A, int64_t nmat_sk,
-                               int64_t m2, int nw) {
-  const int64_t per_w = nmat_sk * m2;
-  const int64_t total = (int64_t)nw * per_w;
-  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
-    int64_t n = e / per_w;
-    int64_t r = e - n * per_w;
-    cplx z = cmk(mu, wn[n]);
-    A[e] = csub(cmul(z, S[r]), X[e]);
-  }
-}
-
-// out[n] = sum_{s,k} w * Tr(A[n][s][k] B[s][k] or B[n][s][k])  (one block per n)
-__global__ void trace_product_kernel(const cplx* A, const cplx* B, bool b_per_w, cplx* out, int64_t nmat_sk, int m,
-                                     double weight) {
-  const int64_t n = blockIdx.x;
-  const int64_t m2 = (int64_t)m * m;
-  const cplx* An = A + n * nmat_sk * m2;
-  const cplx* Bn = b_per_w ? B + n * nmat_sk * m2 : B;
+// tr[n][s,k] = Tr(A[n][s][k] B[n][s][k]), one block per matrix pair
+__global__ void __launch_bounds__(128) trace_product_kernel(const cplx* A, const cplx* B, cplx* tr, int m) {
+  const int64_t mat = blockIdx.x;
+  const int m2 = m * m;
+  const cplx* An = A + mat * m2;
+  const cplx* Bn = B + mat * m2;
   double re = 0.0, im = 0.0;
-  for (int64_t e = threadIdx.x; e < nmat_sk * m2; e += blockDim.x) {
-    int64_t mat = e / m2;
-    int r = (int)(e % m2);
-    int i = r / m, j = r % m;
-    cplx p = cmul(An[mat * m2 + (int64_t)i * m + j], Bn[mat * m2 + (int64_t)j * m + i]);
+  for (int r = threadIdx.x; r < m2; r += 128) {
+    const int i = r / m, j = r - i * m;
+    const cplx p = cmul(An[r], Bn[j * m + i]);
     re += p.x;
     im += p.y;
   }
-  __shared__ double sr[256], si[256];
-  sr[threadIdx.x] = re;
-  si[threadIdx.x] = im;
-  __syncthreads();
-  for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-    if (threadIdx.x < s) {
-      sr[threadIdx.x] += sr[threadIdx.x + s];
-      si[threadIdx.x] += si[threadIdx.x + s];
-    }
-    __syncthreads();
+  __shared__ double sr[4], si[4];
+  for (int o = 16; o > 0; o >>= 1) {
+    re += __shfl_xor_sync(0xffffffffu, re, o);
+    im += __shfl_xor_sync(0xffffffffu, im, o);
   }
-  if (threadIdx.x == 0) out[n] = cmk(sr[0] * weight, si[0] * weight);
+  if (threadIdx.x % 32 == 0) {
+    sr[threadIdx.x / 32] = re;
+    si[threadIdx.x / 32] = im;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) tr[mat] = cmk((sr[0] + sr[1]) + (sr[2] + sr[3]), (si[0] + si[1]) + (si[2] + si[3]));
+}
+
+// out[n] = weight * sum_{s,k} tr[n][s,k], one warp per n
+__global__ void __launch_bounds__(32) trace_sum_kernel(const cplx* tr, cplx* out, int64_t nsk, double weight) {
+  const cplx* t = tr + blockIdx.x * nsk;
+  double re = 0.0, im = 0.0;
+  for (int64_t i = threadIdx.x; i < nsk; i += 32) {
+    re += t[i].x;
+    im += t[i].y;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    re += __shfl_xor_sync(0xffffffffu, re, o);
+    im += __shfl_xor_sync(0xffffffffu, im, o);
+  }
+  if (threadIdx.x == 0) out[blockIdx.x] = cmk(re * weight, im * weight);
 }
 
 // per-(s,k) traces for E_HF, E_1b: out[mat] = (Tr(dm (S1 + 2H)), Tr(dm H)), dm = pref * G(beta)
@@ -150,9 +148,7 @@ void dyson_compute_G(Context& c, cplx* Sigma1, cplx* Sigma_tau, double mu, cplx*
   const int64_t total = (int64_t)d.nw * nsk * m2;
   build_x_kernel<<<grid_for(total, 256), 256, 0, st>>>(c.H.get(), Sigma1, Sw, X, nsk, m2, d.nw);
   GB_CHECK_LAUNCH();
-  build_a_kernel<<<grid_for(total, 256), 256, 0, st>>>(c.S.get(), X, wn, mu, Sw, nsk, m2, d.nw);
-  GB_CHECK_LAUNCH();
-  invert_small_batched(Sw, Gw, (int64_t)d.nw * nsk, d.nso, st);
+  invert_dyson_batched(X, c.S.get(), wn, mu, Gw, d.nw, nsk, d.nso, st);
   ZGemm g;  // G(tau) = Ttn_f G(i w)
   g.M = d.nts; g.N = c.mat_elems(); g.K = d.nw;
   g.A = dense(c.Ttn_f.get(), d.nw);
@@ -180,17 +176,13 @@ void dyson_prepare_X(Context& c, cplx* Sigma1, cplx* Sigma_tau, bool hermitize, 
 double dyson_electrons_prepared(Context& c, double mu, cudaStream_t st) {
   const gb200_dims& d = c.d;
   const int64_t nsk = (int64_t)d.ns * d.nk, m2 = (int64_t)d.nso * d.nso;
-  cplx* A = (cplx*)c.scratch.get(SL_DY_SW, (size_t)d.nw * nsk * m2 * sizeof(cplx));
   cplx* X = (cplx*)c.scratch.get(SL_DY_X, (size_t)d.nw * nsk * m2 * sizeof(cplx));
-  cplx* Gw = (cplx*)c.scratch.get(SL_DY_GW, (size_t)d.nw * nsk * m2 * sizeof(cplx));
+  cplx* tr = (cplx*)c.scratch.get(SL_DY_TR, (size_t)d.nw * nsk * sizeof(cplx));
   double* wn = device_wn(c, st);
   cplx* red = device_red(c);
-  const int64_t total = (int64_t)d.nw * nsk * m2;
-  build_a_kernel<<<grid_for(total, 256), 256, 0, st>>>(c.S.get(), X, wn, mu, A, nsk, m2, d.nw);
-  GB_CHECK_LAUNCH();
-  invert_small_batched(A, Gw, (int64_t)d.nw * nsk, d.nso, st);
-  // trace_w[n] = nkpw * sum_{s,k} weight_k Tr[G(i w_n) S]   (weight 1, nkpw = 1/nk)
-  trace_product_kernel<<<d.nw, 256, 0, st>>>(Gw, c.S.get(), false, red, nsk, d.nso, 1.0 / d.nk);
+  // trace_w[n] = nkpw * sum_{s,k} weight_k Tr[G(i w_n) S]   (weight 1, nkpw = 1/nk); the inverse is not stored
+  trace_dyson_batched(X, c.S.get(), wn, mu, tr, d.nw, nsk, d.nso, st);
+  trace_sum_kernel<<<d.nw, 32, 0, st>>>(tr, red, nsk, 1.0 / d.nk);
   GB_CHECK_LAUNCH();
   std::vector<cplx> tw(d.nw);
   GB_CUDA(cudaMemcpyAsync(tw.data(), red, d.nw * sizeof(cplx), cudaMemcpyDeviceToHost, st));
@@ -254,7 +246,11 @@ void energy(Context& c, const cplx* G, const cplx* Sigma1, const cplx* Sigma_tau
   tau_to_omega(c, G, Gw, st);
   tau_to_omega(c, Sigma_tau, Sw, st);
   cplx* red = device_red(c);
-  trace_product_kernel<<<d.nw, 256, 0, st>>>(Gw, Sw, true, red, nsk, d.nso, 1.0);
+  cplx* tr = (cplx*)c.scratch.get(SL_DY_TR, (size_t)d.nw * nsk * sizeof(cplx));
+  require((int64_t)d.nw * nsk < 2147483647LL, GB200_ERR_INVALID, "energy: too many matrices");
+  trace_product_kernel<<<(unsigned)(d.nw * nsk), 128, 0, st>>>(Gw, Sw, tr, d.nso);
+  GB_CHECK_LAUNCH();
+  trace_sum_kernel<<<d.nw, 32, 0, st>>>(tr, red, nsk, 1.0);
   GB_CHECK_LAUNCH();
   double* h2 = (double*)(red + d.nw);
   const double dm_pref = (d.ns == 2 || c.x2c()) ? -1.0 : -2.0;  // common_utils.cpp:18

@@ -434,7 +434,7 @@ struct GwRun {
       f.C.ptr = Pw; f.C.row = lin((int64_t)NQ * NQ); f.C.col = lin(1);
       zgemm_fp64(f, st);
       // temp = LDLT(I - Pw)^-1 on the lower triangle, then hermitize
-      invert_large_batched(Pw, Pinv, aug, nw_b, NQ, true, true, st);
+      invert_large_batched(Pw, Pinv, aug, (int*)c.scratch.get(SL_INV_BAD, (size_t)nw_b * sizeof(int)), nw_b, NQ, true, st);
       hermitize_batched(Pinv, nw_b, NQ, 1.0, st);
       ZGemm m;  // Pw[n] <- temp[n] Pw[n] (written to aug as scratch, then used)
       m.M = NQ; m.N = NQ; m.K = NQ; m.nb2 = nw_b;

@@ -203,7 +203,7 @@ void gw_sigma_vjp(Context& c, const cplx* G, const cplx* Sb, cplx* Gb, cplx* Vb,
       f.B = dense(P0, nq2);
       f.C.ptr = Pw; f.C.row = lin(nq2); f.C.col = lin(1);
       zgemm_fp64(f, st);
-      invert_large_batched(Pw, T, aug, nw_b, NQ, true, true, st);
+      invert_large_batched(Pw, T, aug, (int*)c.scratch.get(SL_INV_BAD, (size_t)nw_b * sizeof(int)), nw_b, NQ, true, st);
       GB_CUDA(cudaMemcpyAsync(Th, T, (size_t)nw_b * nq2 * sizeof(cplx), cudaMemcpyDeviceToDevice, st));
       hermitize_batched(Th, nw_b, NQ, 1.0, st);
       ZGemm m;  // Ptw = Th Pw
