@@ -736,10 +736,33 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
   } else if (warp == 1) {
     if (lane == 0) {
       int64_t it = 0, tcount = 0;
+      // Slice plane s of A meets the S - s first planes of B at once: they lie one after another in the stage, and
+      // their products belong to the consecutive diagonals s .. S - 1, so they are one MMA of (S - s) BN columns (two
+      // when that is above 256).  For S = 5 and 96 columns a 32-byte K step is 8 MMAs that run at the tensor pipe's
+      // 8192 multiply-adds a cycle; one MMA per pair of planes (15 of 96 columns) is bound by the shared-memory reads
+      // of its operands (56 cycles for 48 of work) and by the issuing thread's descriptor arithmetic.
+      // The descriptors' upper halves and the widths are fixed per tile; per stage only base addresses are added.
+      const uint32_t desc_hi = (uint32_t)(smem_desc_sw64(0) >> 32);
+      const uint32_t ring_lo = (uint32_t)smem_desc_sw64(smem_u32(tiles));
+      const uint32_t stage_lo = (uint32_t)L.stage_bytes >> 4, plane_lo = (uint32_t)L.a_plane_bytes >> 4;
+      uint32_t id0[S], id1[S], dcol1[S], boff1[S];  // per A plane: instruction descriptors of the two parts, and the
+                                                    // second part's column and B row offsets (id1 = 0: one part)
+      int last_bn = 0;
       for (int64_t t = blockIdx.x; t < ntiles && !*abort_flag; t += gridDim.x, ++tcount) {
         const TileRef tr = tile_ref<GROUPED>(p, &mapA, &mapB, t);
         const int tbn = tr.p->BN, nkb = tr.p->nkb;
-        const uint32_t idesc = idesc_i8(tbn);
+        if (tbn != last_bn) {
+          last_bn = tbn;
+#pragma unroll
+          for (int s = 0; s < S; ++s) {
+            const int n = (S - s) * tbn;
+            const int n0 = n <= 256 ? n : (n / 2 + 15) / 16 * 16;
+            id0[s] = idesc_i8(n0);
+            id1[s] = n > n0 ? idesc_i8(n - n0) : 0u;
+            dcol1[s] = (uint32_t)n0;
+            boff1[s] = (uint32_t)(n0 * KBLK) >> 4;
+          }
+        }
         const int buf = (int)(tcount % nbuf);
         const int64_t use = tcount / nbuf;
         if (use > 0 && !mbar_wait(&acce_bar[buf], (uint32_t)((use - 1) & 1), abort_flag)) {
@@ -760,16 +783,17 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
             break;
           }
           tc_fence_after();
-          uint8_t* sbase = tiles + (size_t)st * L.stage_bytes;
-          uint8_t* bbase = sbase + S * L.a_plane_bytes;
-          for (int s = 0; s < S; ++s) {
-            const uint64_t ad = smem_desc_sw64(smem_u32(sbase + s * L.a_plane_bytes));
-            for (int u = 0; s + u < S; ++u) {
-              const uint64_t bd = smem_desc_sw64(smem_u32(bbase + u * tbn * KBLK));
-              const uint32_t dt = acc + (uint32_t)((s + u) * tbn);
+          const uint32_t a_lo = ring_lo + (uint32_t)st * stage_lo, b_lo = a_lo + (uint32_t)S * plane_lo;
 #pragma unroll
-              for (int kk = 0; kk < KBLK / 32; ++kk)
-                umma_i8(dt, ad + 2 * kk, bd + 2 * kk, idesc, (kb > 0 || kk > 0 || s > 0) ? 1u : 0u);
+          for (int kk = 0; kk < KBLK / 32; ++kk) {
+            const uint64_t bd = ((uint64_t)desc_hi << 32) | (b_lo + 2 * kk);
+#pragma unroll
+            for (int s = 0; s < S; ++s) {
+              const uint64_t ad = ((uint64_t)desc_hi << 32) | (a_lo + (uint32_t)s * plane_lo + 2 * kk);
+              const uint32_t dt = acc + (uint32_t)(s * tbn);
+              const uint32_t accum = (kb > 0 || kk > 0 || s > 0) ? 1u : 0u;
+              umma_i8(dt, ad, bd, id0[s], accum);
+              if (id1[s]) umma_i8(dt + dcol1[s], ad, bd + boff1[s], id1[s], accum);
             }
           }
           umma_commit(&empty_bar[st]);
