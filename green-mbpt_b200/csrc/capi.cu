@@ -236,8 +236,7 @@ int gb200_set_grid(gb200_context* ctx, const double* Tnt_f, const double* Ttn_f,
     c.wsample_f.assign(wsample_f, wsample_f + d.nw);
     const cplx* tb = reinterpret_cast<const cplx*>(Ttn_f) + (size_t)(d.nts - 1) * d.nw;
     c.Ttn_beta.assign(tb, tb + d.nw);
-    const cplx* tbb = reinterpret_cast<const cplx*>(Ttn_b);
-    c.Ttn_b_host.assign(tbb, tbb + (size_t)d.nts * d.nw_b);
+    build_w_transforms(c, reinterpret_cast<const cplx*>(Tnt_b), reinterpret_cast<const cplx*>(Ttn_b));
     GB_CUDA(cudaStreamSynchronize(c.stream));
     c.have_grid = true;
   });

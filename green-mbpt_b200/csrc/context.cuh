@@ -57,7 +57,7 @@ enum ScratchSlot {
   SL_IO_S1, SL_IO_H, SL_DM, SL_PINV, SL_SPLIT0, SL_HF_TAB, SL_X2C_DM, SL_X2C_S, SL_X2C_F, SL_X2C_GAB, SL_X2C_GBA,
   SL_X2C_SIG, SL_Q0_Y, SL_Q0_T, SL_Q0_D, SL_Q0_E, SL_Q0_S, SL_ADJ_TH, SL_ADJ_PTW, SL_ADJ_W, SL_ADJ_WB,
   SL_ADJ_PTWB, SL_ADJ_PWB, SL_ADJ_THB, SL_ADJ_XB, SL_ADJ_AB, SL_ADJ_P0B, SL_ADJ_P0HB, SL_ADJ_X3, SL_ADJ_TAB, SL_ADJ_TQ, SL_ADJ_VBF, SL_ADJ_VBH,
-  SL_SINK, SL_INV_BAD, SL_DY_TR, SL_COUNT
+  SL_INV_BAD, SL_DY_TR, SL_SIG_FOLD, SL_COUNT
 };
 
 struct SplitEngine;
@@ -98,7 +98,19 @@ struct Context {
   DevArray<cplx> Tnt_f, Ttn_f, Tnt_b, Ttn_b;
   std::vector<double> wsample_f;
   std::vector<cplx> Ttn_beta;  // host copy of the tau = beta row of Ttn_f
-  std::vector<cplx> Ttn_b_host;  // host copy of Ttn_b [nts][nw_b]
+  // The bosonic transforms as the q loop applies them.  P0(tau) is mirrored exactly (P0(beta - tau) = P0(tau)), so the
+  // forward one is folded onto the first half of tau.  `exact` keeps every frequency and time.  `mirror` also merges
+  // frequencies whose folded rows agree (+-Omega) and gives W on the first half of tau only: usable when the given
+  // matrices are mirror symmetric to well below a contraction's slice rounding (build_w_transforms).
+  struct WTransforms {
+    int nu = 0;            // frequencies
+    int nt = 0;            // times of W: nts, or nts / 2 with W(beta - tau) = W(tau)
+    DevArray<cplx> fwd;    // [nu][nts / 2]
+    DevArray<cplx> bwd;    // [nt][nu]
+    std::vector<cplx> bwd_host;  // [nts][nu]
+  };
+  WTransforms w_exact, w_mirror;  // w_mirror.nu = 0: the grid has no such symmetry
+  DevArray<int64_t> tab_x_mirror; // rows (t, s) of X in mirror-pair order: element offset of (t, s)
   // q -> 0 correction ("extrapolate" treatment, mbpt_q0_utils_t): AqQ [nk][NQ] on the device,
   // |q| on the host, the Madelung constant; eps_inv [nw_b][nk] collects the heads of P(i Omega, q)
   bool q0_on = false;
@@ -148,6 +160,8 @@ struct Context {
 };
 
 // stages implemented in the .cu files
+// the transforms of the q loop from the host matrices Tnt_b [nw_b][nts] and Ttn_b [nts][nw_b]
+void build_w_transforms(Context& c, const cplx* Tnt_b, const cplx* Ttn_b);
 void build_tables(Context& c);
 void build_subset_tables(Context& c);
 // GB200_ERR_STATE unless V holds every pair the q-points [q0, q1) read: (k, k+q) and (k, k-q)

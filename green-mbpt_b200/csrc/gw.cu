@@ -8,9 +8,12 @@
 //  * the three ZGEMMs per (q,k,tau) of P0_contraction (:200-215) and
 //    selfenergy_contraction (:359-373) become three batched GEMMs each:
 //      P0:    T1 = V G(tau,k+q);  Bt = Gbar(beta-tau,k) T1;  P0 -= pref Bt . conj(V)
-//      Sigma: Y1 = V G(tau,k-q);  Y2 = Y1^T W(tau);           Sigma -= Y2 . conj(V)
+//      Sigma: X = G(tau,k-q) V^H; Z = V W(tau);               Sigma -= Z . X
 //    which is the same sum, P0_QQ' = -pref sum Gbar_tp V^Q_pm G_mn conj(V^Q'_tn),
-//    Sigma_ij = -sum V^Q_im G_mn W_QQ' conj(V^Q'_jn), in a batched order.
+//    Sigma_ij = -sum V^Q_im G_mn W_QQ' conj(V^Q'_jn), in a batched order.  Z, the contraction over the square
+//    of the auxiliary basis, needs neither the spin nor, where W(beta - tau) = W(tau), the second half of
+//    tau.  With one spin and no such symmetry it saves nothing, and the sum runs as
+//      Sigma: Y1 = V G(tau,k-q);  Y2 = Y1^T W(tau);           Sigma -= Y2 . conj(V).
 #include <algorithm>
 #include <cmath>
 #include <memory>
@@ -22,7 +25,8 @@
 namespace gb200 {
 namespace {
 
-// P0(t) = herm(P0(t)/nk), P0(nts-1-t) = P0(t) for t < nts/2 (gw_cpu_kernel.cpp:217-225).
+// P0(t) = herm(P0(t)/nk) for t < nts/2, from its transpose in place (gw_cpu_kernel.cpp:217-225; the mirrored half is
+// never formed).
 __global__ void symmetrize_p0_kernel(cplx* P0, int nts, int NQ, double inv_nk) {
   const int nth = nts / 2;
   const int64_t npairs = (int64_t)NQ * (NQ + 1) / 2;
@@ -35,14 +39,11 @@ __global__ void symmetrize_p0_kernel(cplx* P0, int nts, int NQ, double inv_nk) {
     while ((int64_t)(i + 1) * (i + 2) / 2 <= p) ++i;
     int j = (int)(p - (int64_t)i * (i + 1) / 2);
     cplx* M = P0 + (int64_t)t * NQ * NQ;
-    cplx* Mm = P0 + (int64_t)(nts - 1 - t) * NQ * NQ;
-    cplx a = cscale(M[(int64_t)i * NQ + j], inv_nk);
-    cplx b = cscale(M[(int64_t)j * NQ + i], inv_nk);
+    cplx a = cscale(M[(int64_t)j * NQ + i], inv_nk);
+    cplx b = cscale(M[(int64_t)i * NQ + j], inv_nk);
     cplx h = cscale(cadd(a, cconj(b)), 0.5);
     M[(int64_t)i * NQ + j] = h;
     M[(int64_t)j * NQ + i] = cconj(h);
-    Mm[(int64_t)i * NQ + j] = h;
-    Mm[(int64_t)j * NQ + i] = cconj(h);
   }
 }
 
@@ -99,6 +100,16 @@ __global__ void q0_x2c_offdiag_kernel(cplx* D, int64_t nmat, int n) {
     const int64_t m = e / n2, r = e % n2, i = r / n, j = r % n;
     cplx* M = D + m * so * so;
     M[(j + n) * so + i] = cconj(M[i * so + (j + n)]);
+  }
+}
+
+// Sigma[t][..] = scale * F[..] with F in mirror pairs: F[2 t] is time t, F[2 t + 1] time nts - 1 - t
+__global__ void unfold_sigma_kernel(const cplx* F, cplx* Sigma, int nts, int64_t per_t, double scale) {
+  const int64_t total = (int64_t)nts * per_t;
+  for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < total; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t t = e / per_t, r = e - t * per_t;
+    const int64_t f = 2 * t < nts ? 2 * t : 2 * (nts - 1 - t) + 1;
+    Sigma[e] = cscale(F[f * per_t + r], scale);
   }
 }
 
@@ -171,11 +182,92 @@ void build_subset_tables(Context& c) {
   GB_CUDA(cudaStreamSynchronize(c.stream));
 }
 
-// Choose the k-block size so that the two largest intermediates fit the budget.
-static int choose_kblock(const Context& c, int64_t elems_per_k) {
-  // leave headroom; at most 24 GB for the GW intermediates unless the caller set a budget
-  const double budget = c.budget_or(24e9, 0.6);
-  double per_k = 2.0 * (double)elems_per_k * sizeof(cplx);
+// The largest mirror asymmetry of the transforms, relative to their largest element, at which the folded form is used:
+// 2^-39, the unit in which five slices hold an operand.  (The synthetic Chebyshev grids have
+// 1e-13 to 5e-13, so FP64 and six slices keep the matrices as given.)
+constexpr double MIRROR_TOL = 1.8e-12;
+constexpr int MIRROR_MAX_SLICES = 5;
+
+void build_w_transforms(Context& c, const cplx* Tnt, const cplx* Ttn) {
+  const int nts = c.d.nts, nth = nts / 2, nw = c.d.nw_b, ns = c.ns_eff();
+  std::vector<cplx> fold((size_t)nw * nth);
+  double fmax = 0.0, bmax = 0.0;
+  for (int n = 0; n < nw; ++n)
+    for (int t = 0; t < nth; ++t) {
+      const cplx v = cadd(Tnt[(size_t)n * nts + t], Tnt[(size_t)n * nts + nts - 1 - t]);
+      fold[(size_t)n * nth + t] = v;
+      fmax = std::max(fmax, std::max(std::fabs(v.x), std::fabs(v.y)));
+    }
+  Context::WTransforms& e = c.w_exact;
+  e.nu = nw;
+  e.nt = nts;
+  e.fwd.upload(fold.data(), fold.size(), c.stream);
+  e.bwd.upload(Ttn, (size_t)nts * nw, c.stream);
+  e.bwd_host.assign(Ttn, Ttn + (size_t)nts * nw);
+  // frequencies with equal folded rows (each joins the first such one)
+  std::vector<int> group(nw, -1), first;
+  for (int n = 0; n < nw; ++n) {
+    for (size_t u = 0; u < first.size() && group[n] < 0; ++u) {
+      bool same = true;
+      for (int t = 0; same && t < nth; ++t) {
+        const cplx a = fold[(size_t)n * nth + t], b = fold[(size_t)first[u] * nth + t];
+        same = std::fabs(a.x - b.x) <= MIRROR_TOL * fmax && std::fabs(a.y - b.y) <= MIRROR_TOL * fmax;
+      }
+      if (same) group[n] = (int)u;
+    }
+    if (group[n] < 0) {
+      group[n] = (int)first.size();
+      first.push_back(n);
+    }
+  }
+  const int nu = (int)first.size();
+  std::vector<cplx> fwd((size_t)nu * nth, cmk(0.0, 0.0)), full((size_t)nts * nu, cmk(0.0, 0.0)), half((size_t)nth * nu);
+  std::vector<int> members(nu, 0);
+  for (int n = 0; n < nw; ++n) {
+    ++members[group[n]];
+    for (int t = 0; t < nth; ++t) {
+      cplx& f = fwd[(size_t)group[n] * nth + t];
+      f = cadd(f, fold[(size_t)n * nth + t]);
+    }
+    for (int t = 0; t < nts; ++t) {
+      cplx& f = full[(size_t)t * nu + group[n]];
+      f = cadd(f, Ttn[(size_t)t * nw + n]);
+    }
+  }
+  for (int u = 0; u < nu; ++u)
+    for (int t = 0; t < nth; ++t) fwd[(size_t)u * nth + t] = cscale(fwd[(size_t)u * nth + t], 1.0 / members[u]);
+  double asym = 0.0;
+  bool finite = true;
+  for (int t = 0; t < nth; ++t)
+    for (int u = 0; u < nu; ++u) {
+      const cplx a = full[(size_t)t * nu + u], b = full[(size_t)(nts - 1 - t) * nu + u];
+      bmax = std::max(bmax, std::max(std::max(std::fabs(a.x), std::fabs(a.y)), std::max(std::fabs(b.x), std::fabs(b.y))));
+      asym = std::max(asym, std::max(std::fabs(a.x - b.x), std::fabs(a.y - b.y)));
+      finite = finite && std::isfinite(a.x + a.y + b.x + b.y);
+      half[(size_t)t * nu + u] = cscale(cadd(a, b), 0.5);
+    }
+  Context::WTransforms& m = c.w_mirror;
+  m.nu = finite && asym <= MIRROR_TOL * bmax ? nu : 0;
+  if (m.nu > 0) {
+    m.nt = nth;
+    m.fwd.upload(fwd.data(), fwd.size(), c.stream);
+    m.bwd.upload(half.data(), half.size(), c.stream);
+    m.bwd_host = full;
+    std::vector<int64_t> tab((size_t)nts * ns);
+    for (int t = 0; t < nts; ++t)
+      for (int s = 0; s < ns; ++s)
+        tab[(size_t)t * ns + s] = ((int64_t)(t < nth ? 2 * t : 2 * (nts - 1 - t) + 1) * ns + s) * c.pair_elems();
+    c.tab_x_mirror.upload(tab.data(), tab.size(), c.stream);
+  }
+  GB_CUDA(cudaStreamSynchronize(c.stream));
+}
+
+// Choose the k-block size so that the intermediates (and, without a caller's budget, the slice planes of the largest
+// contraction) fit the budget.
+static int choose_kblock(const Context& c, int64_t elems_per_k, int64_t plane_bytes_per_k) {
+  // leave headroom; at most 24 GB for the GW intermediates (40 GB with their planes) unless the caller set a budget
+  const double budget = c.budget_or(plane_bytes_per_k > 0 ? 40e9 : 24e9, 0.6);
+  double per_k = (double)elems_per_k * sizeof(cplx) + (c.mem_budget > 0.0 ? 0.0 : (double)plane_bytes_per_k);
   int kb = (int)std::max(1.0, std::floor(budget / per_k));
   return std::min(kb, c.d.nk);
 }
@@ -237,10 +329,10 @@ cplx extrapolate_q0(const cplx* eps_n, const std::vector<double>& q_abs, int fit
 }
 
 // Sigma += -madelung eps_inv_q0(t) S G(t) S (GW_q0_correction, mbpt_q0_utils_t.cpp:88-178)
-static void apply_q0(Context& c, const cplx* G, cplx* Sigma, cudaStream_t st) {
+static void apply_q0(Context& c, const Context::WTransforms& wt, const cplx* G, cplx* Sigma, cudaStream_t st) {
   const gb200_dims& d = c.d;
   require(c.have_H, GB200_ERR_STATE, "q0 correction: the overlap (gb200_dyson_set_hamiltonian) must be set");
-  const int nk = d.nk, nts = d.nts, nw_b = d.nw_b;
+  const int nk = d.nk, nts = d.nts, nw_b = wt.nu;
   const int64_t nso = d.nso, m2 = nso * nso, nmat = (int64_t)d.ns * nk;
   std::vector<cplx> eps((size_t)nw_b * nk);
   GB_CUDA(cudaMemcpyAsync(eps.data(), c.eps_inv.get(), eps.size() * sizeof(cplx), cudaMemcpyDeviceToHost, st));
@@ -249,7 +341,7 @@ static void apply_q0(Context& c, const cplx* G, cplx* Sigma, cudaStream_t st) {
   for (int n = 0; n < nw_b; ++n) ew[n] = extrapolate_q0(eps.data() + (size_t)n * nk, c.q_abs, 2, 1.0);
   for (int t = 0; t < nts; ++t) {
     cplx acc = cmk(0.0, 0.0);
-    for (int n = 0; n < nw_b; ++n) acc = cadd(acc, cmul(c.Ttn_b_host[(size_t)t * nw_b + n], ew[n]));
+    for (int n = 0; n < nw_b; ++n) acc = cadd(acc, cmul(wt.bwd_host[(size_t)t * nw_b + n], ew[n]));
     coef[t] = cscale(acc, -c.q0_madelung);
   }
   cplx* dcoef = (cplx*)c.scratch.get(SL_Q0_E, (size_t)nts * sizeof(cplx));
@@ -306,17 +398,13 @@ struct GwRun {
   const cplx* Gbar;  // the operand of Gbar(beta - tau, k): block (b,a) for two-component input
   cplx* Sigma;
   int kb = 1;
-  int64_t per_k_sigma = 0;
+  // Sigma through Z = V W and X = G V^H (else through Y1 and Y2): nh times share a Z, ntz times have one
+  const Context::WTransforms* wt = nullptr;
+  bool by_z = false;
+  int nh = 1, ntz = 0;
+  cplx* acc = nullptr;  // what the q loop accumulates: Sigma, in mirror pairs of times when nh = 2
   cplx *P0 = nullptr, *Pw = nullptr, *Pinv = nullptr, *aug = nullptr, *X1 = nullptr, *X2 = nullptr;
   int q0 = 0, q1 = 0;
-  // exponent sink (split precision on the tensor cores): (e) records the column exponents of Y2
-  // for (f) as it stores Y2, so that slicing Y2 needs no separate exponent pass.  Measured on the
-  // c2 shapes it costs (e) about 0.4 of the pass it saves; in the epilogue-bound (b) it would cost
-  // more than the pass for Bt, so (b) -> (c) keeps the pass.
-  bool sink_s = false;
-  int32_t* sink = nullptr;
-  int64_t sink_ld_s = 0;
-
   GwRun(Context& c_, const cplx* G_, cplx* Sigma_, cudaStream_t st_) : c(c_), st(st_), d(c_.d) {
     require(d.nts % 2 == 0, GB200_ERR_WRONG_GRID, "Number of tau points should be even!!!");
     require(c.have_kq && c.have_grid && c.have_V, GB200_ERR_STATE, "gw_sigma: k/q maps, grid and integrals must be set");
@@ -345,21 +433,28 @@ struct GwRun {
       Gbar = Gba;
       Sigma = (cplx*)c.scratch.get(SL_X2C_SIG, (size_t)n * sizeof(cplx));
     }
-    GB_CUDA(cudaMemsetAsync(Sigma, 0, (size_t)nts * ns * nk * nao2 * sizeof(cplx), st));
-    per_k_sigma = (int64_t)nts * ns * pe;
-    kb = choose_kblock(c, per_k_sigma);
+    auto slices_of = [&](int stage) { return c.contraction_slices[stage] > 0 ? c.contraction_slices[stage] : c.slices; };
+    const bool split = c.prec_mode == GB200_PREC_SPLIT;
+    int smin = 8;  // the coarsest contraction sets the error
+    for (int i = 0; i < 6; ++i) smin = std::min(smin, slices_of(i));
+    wt = split && smin <= MIRROR_MAX_SLICES && c.w_mirror.nu > 0 ? &c.w_mirror : &c.w_exact;
+    ntz = wt->nt;
+    nh = nts / ntz;
+    by_z = nh * ns > 1;
+    acc = nh == 2 ? (cplx*)c.scratch.get(SL_SIG_FOLD, (size_t)nts * ns * nk * nao2 * sizeof(cplx)) : Sigma;
+    GB_CUDA(cudaMemsetAsync(acc, 0, (size_t)nts * ns * nk * nao2 * sizeof(cplx), st));
+    const int64_t x1_k = (int64_t)nts * ns * pe;
+    const int64_t x2_k = by_z ? std::max((int64_t)nth * ns, (int64_t)ntz) * pe : x1_k;
+    // planes of (f): 2 bytes a slice and element of the right operand, 4 of the left one
+    const int64_t planes_k = !split ? 0 : 2 * slices_of(5) * (by_z ? x1_k + 2 * (int64_t)ntz * pe : x1_k);
+    kb = choose_kblock(c, x1_k + x2_k, planes_k);
+    kb = std::min<int64_t>(kb, std::max<int64_t>(1, 65535 / ((int64_t)nts * ns)));  // batches of one launch
     P0 = (cplx*)c.scratch.get(SL_P0, (size_t)nts * NQ * NQ * sizeof(cplx));
     Pw = (cplx*)c.scratch.get(SL_PW, (size_t)nw_b * NQ * NQ * sizeof(cplx));
     Pinv = (cplx*)c.scratch.get(SL_PINV, (size_t)nw_b * NQ * NQ * sizeof(cplx));
     aug = (cplx*)c.scratch.get(SL_AUG, (size_t)nw_b * NQ * 2 * NQ * sizeof(cplx));
-    X1 = (cplx*)c.scratch.get(SL_Y1, (size_t)kb * per_k_sigma * sizeof(cplx));
-    X2 = (cplx*)c.scratch.get(SL_Y2, (size_t)kb * per_k_sigma * sizeof(cplx));
-    if (c.prec_mode == GB200_PREC_SPLIT && c.split_core == 0 && nao % 8 == 0) {
-      auto slices_of = [&](int stage) { return c.contraction_slices[stage] > 0 ? c.contraction_slices[stage] : c.slices; };
-      sink_s = NQ <= split_max_chunk(slices_of(4));
-      sink_ld_s = (int64_t)nts * ns * nao;
-      if (sink_s) sink = (int32_t*)c.scratch.get(SL_SINK, (size_t)kb * sink_ld_s * sizeof(int32_t));
-    }
+    X1 = (cplx*)c.scratch.get(SL_Y1, (size_t)kb * x1_k * sizeof(cplx));
+    X2 = (cplx*)c.scratch.get(SL_Y2, (size_t)kb * x2_k * sizeof(cplx));
     if (c.q0_on) {
       require(c.q_begin <= 0 && (c.q_end < 0 || c.q_end >= nk), GB200_ERR_INVALID,
               "q0 correction: needs all q-points in one context (it extrapolates over q)");
@@ -382,15 +477,15 @@ struct GwRun {
     const int64_t* tVp = c.tab_pair_plus.get() + (int64_t)q * nk + k0;
     const int64_t* tGp = c.tab_g_plus.get() + (int64_t)q * nk + k0;
     const int64_t blkT1 = (int64_t)nth * ns * pe;  // per kk in T1
-      // (a) T1[kk][t][s][(Q,p)][n] = sum_m V(k,k+q)[(Q,p)][m] G(t,s,k+q)[m][n], computed as its
-    //     transpose T1^T = G^T V^T so that the large operand V is the right (column) operand:
-    //     rows ((t,s),n) (M = nth*ns*nao), columns (Q,p) (N = NQ*nao), K = m
+    // (a) T1[kk][t][s][n][(Q,p)] = sum_m V(k,k+q)[(Q,p)][m] G(t,s,k+q)[m][n], as G^T V^T so that the large
+    //     operand V is the right (column) operand: rows ((t,s),n) (M = nth*ns*nao), columns (Q,p)
+    //     (N = NQ*nao, unit stride in T1), K = m
     ZGemm a;
     a.M = (int64_t)nth * ns * nao; a.N = (int64_t)NQ * nao; a.K = nao;
     a.nb0 = kbk;
     a.A.ptr = G; a.A.row = two(nao, 1, g_s); a.A.col = lin(nao); a.A.bat.tab0 = tGp;
     a.B.ptr = c.V.get(); a.B.row = lin(1); a.B.col = lin(nao); a.B.bat.tab0 = tVp;
-    a.C.ptr = X1; a.C.row = two(nao, 1, pe); a.C.col = lin(nao);
+    a.C.ptr = X1; a.C.row = two(nao, (int64_t)NQ * nao, pe); a.C.col = lin(1);
     a.C.bat.s0 = blkT1;
     // (b) Bt[t][kk][s][Q][r][n] = sum_p Gbar(nts-1-t, s, k)[r][p] T1[kk][t][s][Q][p][n]
     ZGemm b;
@@ -398,13 +493,14 @@ struct GwRun {
     b.nb0 = kbk; b.nb1 = nth; b.nb2 = ns;
     b.A = dense(Gbar + (int64_t)(nts - 1) * g_t + (int64_t)k0 * ge, nao);
     b.A.bat.s0 = ge; b.A.bat.s1 = -g_t; b.A.bat.s2 = g_s;
-    b.B.ptr = X1; b.B.row = lin(nao); b.B.col = two(nao, 1, nao2);
+    b.B.ptr = X1; b.B.row = lin(1); b.B.col = two(nao, (int64_t)NQ * nao, nao);
     b.B.bat.s0 = blkT1; b.B.bat.s1 = (int64_t)ns * pe; b.B.bat.s2 = pe;
     b.C.ptr = X2; b.C.row = lin(nao); b.C.col = two(nao, 1, nao2);
     b.C.bat.s0 = (int64_t)ns * pe; b.C.bat.s1 = (int64_t)kbk * ns * pe; b.C.bat.s2 = pe;
     // (c) P0[t][Q][Q'] -= pref sum_{(kk,s),(r,n)} Bt[t][(kk,s)][Q][(r,n)] conj(V(k,k+q)[Q'][(r,n)]),
     //     computed as P0^T = conj(V) Bt^T: the tau-independent V is the left operand (sliced
-    //     once per call), Bt the right one; rows Q', columns Q, K = ((kk,s),(r,n))
+    //     once per call), Bt the right one; rows Q', columns Q, K = ((kk,s),(r,n)).  Kept transposed,
+    //     [t][Q'][Q], until w_solve hermitizes it
     ZGemm cc;
     cc.M = NQ; cc.N = NQ; cc.K = (int64_t)kbk * ns * nao2;
     cc.nb0 = 1; cc.nb1 = 1; cc.nb2 = nth;
@@ -412,7 +508,7 @@ struct GwRun {
     cc.A.col = twotab(nao2, 1, c.tab_pair_plus_ns.get() + ((int64_t)q * nk + k0) * ns);
     cc.B.ptr = X2; cc.B.col = lin(nao2); cc.B.row = two(nao2, 1, (int64_t)NQ * nao2);
     cc.B.bat.s2 = (int64_t)kbk * ns * pe;
-    cc.C.ptr = P0; cc.C.row = lin(1); cc.C.col = lin(NQ); cc.C.bat.s2 = (int64_t)NQ * NQ;
+    cc.C.ptr = P0; cc.C.row = lin(NQ); cc.C.col = lin(1); cc.C.bat.s2 = (int64_t)NQ * NQ;
     cc.alpha = cmk(-pref, 0.0); cc.beta = cmk(1.0, 0.0);
     out[0] = a;
     out[1] = b;
@@ -421,23 +517,24 @@ struct GwRun {
 
   // ---------------- screened interaction (gw_cpu_kernel.cpp:227-279) -------
   void w_solve(int q) {
-    {  // P0 = herm(P0 / nk), P0(beta - tau) = P0(tau) (gw_cpu_kernel.cpp:217-225)
+    const int nu = wt->nu;
+    {  // P0 = herm(P0 / nk); P0(beta - tau) = P0(tau) (gw_cpu_kernel.cpp:217-225) is in the folded transform
       int64_t total = (int64_t)nth * NQ * (NQ + 1) / 2;
       symmetrize_p0_kernel<<<grid_for(total, 256), 256, 0, st>>>(P0, nts, NQ, 1.0 / nk);
       GB_CHECK_LAUNCH();
     }
     {
       ZGemm f;  // Pw[n] = sum_t Tnt_b[n][t] P0[t]
-      f.M = nw_b; f.N = (int64_t)NQ * NQ; f.K = nts;
-      f.A = dense(c.Tnt_b.get(), nts);
+      f.M = nu; f.N = (int64_t)NQ * NQ; f.K = nth;
+      f.A = dense(wt->fwd.get(), nth);
       f.B = dense(P0, (int64_t)NQ * NQ);
       f.C.ptr = Pw; f.C.row = lin((int64_t)NQ * NQ); f.C.col = lin(1);
       zgemm_fp64(f, st);
       // temp = LDLT(I - Pw)^-1 on the lower triangle, then hermitize
-      invert_large_batched(Pw, Pinv, aug, (int*)c.scratch.get(SL_INV_BAD, (size_t)nw_b * sizeof(int)), nw_b, NQ, true, st);
-      hermitize_batched(Pinv, nw_b, NQ, 1.0, st);
+      invert_large_batched(Pw, Pinv, aug, (int*)c.scratch.get(SL_INV_BAD, (size_t)nw_b * sizeof(int)), nu, NQ, true, st);
+      hermitize_batched(Pinv, nu, NQ, 1.0, st);
       ZGemm m;  // Pw[n] <- temp[n] Pw[n] (written to aug as scratch, then used)
-      m.M = NQ; m.N = NQ; m.K = NQ; m.nb2 = nw_b;
+      m.M = NQ; m.N = NQ; m.K = NQ; m.nb2 = nu;
       m.A = dense(Pinv, NQ); m.A.bat.s2 = (int64_t)NQ * NQ;
       m.B = dense(Pw, NQ); m.B.bat.s2 = (int64_t)NQ * NQ;
       m.C.ptr = aug; m.C.row = lin(NQ); m.C.col = lin(1); m.C.bat.s2 = (int64_t)NQ * NQ;
@@ -448,21 +545,21 @@ struct GwRun {
         cplx* y = (cplx*)c.scratch.get(SL_Q0_Y, (size_t)nw_b * NQ * sizeof(cplx));
         const cplx* Aq = c.AqQ.get() + (int64_t)q * NQ;
         ZGemm hy;  // y[n][Q] = sum_Q' P[n][Q][Q'] A_q[Q']
-        hy.M = NQ; hy.N = 1; hy.K = NQ; hy.nb2 = nw_b;
+        hy.M = NQ; hy.N = 1; hy.K = NQ; hy.nb2 = nu;
         hy.A = dense(aug, NQ); hy.A.bat.s2 = (int64_t)NQ * NQ;
         hy.B.ptr = Aq; hy.B.row = lin(1); hy.B.col = lin(0);
         hy.C.ptr = y; hy.C.row = lin(1); hy.C.col = lin(0); hy.C.bat.s2 = NQ;
         zgemm_fp64(hy, st);
         ZGemm he;  // eps_inv[n][q] = sum_Q conj(A_q[Q]) y[n][Q]
-        he.M = 1; he.N = 1; he.K = NQ; he.nb2 = nw_b;
+        he.M = 1; he.N = 1; he.K = NQ; he.nb2 = nu;
         he.A.ptr = Aq; he.A.row = lin(0); he.A.col = lin(1); he.A.conj = true;
         he.B.ptr = y; he.B.row = lin(1); he.B.col = lin(0); he.B.bat.s2 = NQ;
         he.C.ptr = c.eps_inv.get() + q; he.C.row = lin(0); he.C.col = lin(0); he.C.bat.s2 = nk;
         zgemm_fp64(he, st);
       }
       ZGemm bt;  // W(tau) = sum_n Ttn_b[t][n] P(i Omega_n) -> stored in P0
-      bt.M = nts; bt.N = (int64_t)NQ * NQ; bt.K = nw_b;
-      bt.A = dense(c.Ttn_b.get(), nw_b);
+      bt.M = ntz; bt.N = (int64_t)NQ * NQ; bt.K = nu;
+      bt.A = dense(wt->bwd.get(), nu);
       bt.B = dense(aug, (int64_t)NQ * NQ);
       bt.C.ptr = P0; bt.C.row = lin((int64_t)NQ * NQ); bt.C.col = lin(1);
       zgemm_fp64(bt, st);
@@ -474,60 +571,93 @@ struct GwRun {
     const int kbk = std::min(kb, nk - k0);
     const int64_t* tVm = c.tab_pair_minus.get() + (int64_t)q * nk + k0;
     const int64_t* tGm = c.tab_g_minus.get() + (int64_t)q * nk + k0;
-    const int64_t blk = (int64_t)nts * ns * pe;  // per kk in Y1 / Y2
-      // (d) Y1[kk][t][s][(Q,i)][n] = sum_m V(k,k-q)[(Q,i)][m] G(t,s,k-q)[m][n], as its transpose
-    //     (V the right operand): rows ((t,s),n), columns (Q,i), K = m
+    const int64_t blk = (int64_t)nts * ns * pe;  // per kk in X, Y1 and Y2
+    if (by_z) {
+      const int64_t zblk = (int64_t)ntz * pe;  // per kk in Z
+      // (d) X[kk][t][s][m][(Q',j)] = sum_n conj(V(k,k-q)[Q'][j][n]) G(t,s,k-q)[m][n]: rows ((t,s),m), columns (Q',j),
+      //     K = n; with nh = 2 the times lie in mirror pairs (t, nts-1-t)
+      ZGemm dd;
+      dd.M = (int64_t)nts * ns * nao; dd.N = (int64_t)NQ * nao; dd.K = nao;
+      dd.nb0 = kbk;
+      dd.A.ptr = G; dd.A.row = two(nao, nao, g_s); dd.A.col = lin(1); dd.A.bat.tab0 = tGm;
+      dd.B.ptr = c.V.get(); dd.B.row = lin(1); dd.B.col = lin(nao); dd.B.conj = true; dd.B.bat.tab0 = tVm;
+      dd.C.ptr = X1; dd.C.row = nh == 2 ? twotab(nao, (int64_t)NQ * nao, c.tab_x_mirror.get()) : two(nao, (int64_t)NQ * nao, pe);
+      dd.C.col = lin(1);
+      dd.C.bat.s0 = blk;
+      // (e) Z[kk][t][(i,m)][Q'] = sum_Q V(k,k-q)[Q][(i,m)] W(t)[Q][Q']: rows (i,m), columns Q' (unit stride in Z), K = Q.
+      //     V is sliced once per k and W once per time; both are small beside Z
+      ZGemm e;
+      e.M = nao2; e.N = NQ; e.K = NQ;
+      e.nb0 = kbk; e.nb1 = ntz;
+      e.A.ptr = c.V.get(); e.A.row = lin(1); e.A.col = lin(nao2); e.A.bat.tab0 = tVm;
+      e.B.ptr = P0; e.B.row = lin(NQ); e.B.col = lin(1); e.B.bat.s1 = (int64_t)NQ * NQ;
+      e.C.ptr = X2; e.C.row = lin(NQ); e.C.col = lin(1); e.C.bat.s0 = zblk; e.C.bat.s1 = pe;
+      // (f) Sigma[t][h][s][k][i][j] -= sum_{(m,Q')} Z[kk][t][i][(m,Q')] X[kk][t][h][s][(m,Q')][j]: rows i, columns (h,s,j),
+      //     K = (m,Q'), contiguous in Z and of stride nao in X; one batch per k and Z
+      ZGemm f;
+      f.M = nao; f.N = (int64_t)nh * ns * nao; f.K = (int64_t)NQ * nao;
+      f.nb0 = kbk; f.nb1 = ntz;
+      f.A.ptr = X2; f.A.row = lin((int64_t)NQ * nao); f.A.col = lin(1); f.A.bat.s0 = zblk; f.A.bat.s1 = pe;
+      f.B.ptr = X1; f.B.row = lin(nao); f.B.col = two(nao, 1, pe);
+      f.B.bat.s0 = blk; f.B.bat.s1 = (int64_t)nh * ns * pe;
+      f.C.ptr = acc + (int64_t)k0 * ge; f.C.row = lin(nao); f.C.col = two(nao, 1, g_s);
+      f.C.bat.s0 = ge; f.C.bat.s1 = (int64_t)nh * ns * g_s;
+      f.alpha = cmk(-1.0, 0.0); f.beta = cmk(1.0, 0.0);
+      out[0] = dd;
+      out[1] = e;
+      out[2] = f;
+      return;
+    }
+    // (d) Y1[kk][t][s][n][(Q,i)] = sum_m V(k,k-q)[(Q,i)][m] G(t,s,k-q)[m][n], as G^T V^T (V the right
+    //     operand): rows ((t,s),n), columns (Q,i), K = m
     ZGemm dd;
     dd.M = (int64_t)nts * ns * nao; dd.N = (int64_t)NQ * nao; dd.K = nao;
     dd.nb0 = kbk;
     dd.A.ptr = G; dd.A.row = two(nao, 1, g_s); dd.A.col = lin(nao); dd.A.bat.tab0 = tGm;
     dd.B.ptr = c.V.get(); dd.B.row = lin(1); dd.B.col = lin(nao); dd.B.bat.tab0 = tVm;
-    dd.C.ptr = X1; dd.C.row = two(nao, 1, pe); dd.C.col = lin(nao);
+    dd.C.ptr = X1; dd.C.row = two(nao, (int64_t)NQ * nao, pe); dd.C.col = lin(1);
     dd.C.bat.s0 = blk;
-    // (e) Y2[kk][t][s][(i,n)][Q'] = sum_Q Y1[kk][t][s][Q][(i,n)] W(t)[Q][Q'], as Y2^T = W^T Y1:
-    //     the small W(t) is the left operand, Y1 the right one; rows Q', columns (kk,(i,n)), K = Q
+    // (e) Y2[kk][t][s][Q'][(n,i)] = sum_Q W(t)[Q][Q'] Y1[kk][t][s][n][Q][i]: rows Q', columns (n,i), K = Q
     ZGemm e;
-    e.M = NQ; e.N = (int64_t)kbk * nao2; e.K = NQ;
-    e.nb0 = 1; e.nb1 = nts; e.nb2 = ns;
+    e.M = NQ; e.N = nao2; e.K = NQ;
+    e.nb0 = kbk; e.nb1 = nts; e.nb2 = ns;
     e.A.ptr = P0; e.A.row = lin(1); e.A.col = lin(NQ); e.A.bat.s1 = (int64_t)NQ * NQ;
-    e.B.ptr = X1; e.B.row = lin(nao2); e.B.col = two(nao2, 1, blk);
-    e.B.bat.s1 = (int64_t)ns * pe; e.B.bat.s2 = pe;
-    e.C.ptr = X2; e.C.row = lin(1); e.C.col = two(nao2, NQ, blk);
-    e.C.bat.s1 = (int64_t)ns * pe; e.C.bat.s2 = pe;
-    // (f) Sigma[t][s][k][i][j] -= sum_{(n,Q')} Y2[kk][t][s][i][(n,Q')] conj(V(k,k-q)[Q'][j][n]), as
+    e.B.ptr = X1; e.B.row = lin(nao); e.B.col = two(nao, 1, (int64_t)NQ * nao);
+    e.B.bat.s0 = blk; e.B.bat.s1 = (int64_t)ns * pe; e.B.bat.s2 = pe;
+    e.C.ptr = X2; e.C.row = lin(nao2); e.C.col = lin(1);
+    e.C.bat.s0 = blk; e.C.bat.s1 = (int64_t)ns * pe; e.C.bat.s2 = pe;
+    // (f) Sigma[t][s][k][i][j] -= sum_{(Q',n)} Y2[kk][t][s][Q'][n][i] conj(V(k,k-q)[Q'][j][n]), as
     //     Sigma^T = conj(V) Y2^T: rows j (M = nao), columns ((t,s),i) (N = nts*ns*nao),
-    //     K = (n,Q'); the large Y2 is the right operand
+    //     K = (Q',n); the large Y2 is the right operand
     ZGemm f;
-    f.M = nao; f.N = (int64_t)nts * ns * nao; f.K = nao * NQ;
+    f.M = nao; f.N = (int64_t)nts * ns * nao; f.K = (int64_t)NQ * nao;
     f.nb0 = kbk;
-    f.A.ptr = c.V.get(); f.A.row = lin(nao); f.A.col = two(NQ, nao2, 1); f.A.conj = true;
+    f.A.ptr = c.V.get(); f.A.row = lin(nao); f.A.col = two(nao, 1, nao2); f.A.conj = true;
     f.A.bat.tab0 = tVm;
-    f.B.ptr = X2; f.B.row = lin(1); f.B.col = two(nao, nao * NQ, pe);
+    f.B.ptr = X2; f.B.row = two(nao, nao, nao2); f.B.col = two(nao, 1, pe);
     f.B.bat.s0 = blk;
-    f.C.ptr = Sigma + (int64_t)k0 * ge; f.C.row = lin(1); f.C.col = two(nao, nao, g_s);
+    f.C.ptr = acc + (int64_t)k0 * ge; f.C.row = lin(1); f.C.col = two(nao, nao, g_s);
     f.C.bat.s0 = ge;
     f.alpha = cmk(-1.0, 0.0); f.beta = cmk(1.0, 0.0);
-    if (sink_s) {
-      // column ((t,s),i) of (f)'s B in batch kk: Y2[kk][t][s][i][*], i.e. (e)'s columns
-      // (kk,(i,n)) in its batch (t, s): entry kk ld + (t ns + s) nao + i
-      e.sink.expo = sink; e.sink.c1 = (int64_t)ns * nao; e.sink.c2 = nao;
-      e.sink.d1 = nao; e.sink.m1 = nao; e.sink.s1 = 1; e.sink.d2 = nao2; e.sink.s2 = sink_ld_s;
-      e.sink.count = (int64_t)kbk * sink_ld_s;
-      f.B_expo = sink; f.B_expo_ld = sink_ld_s;
-    }
     out[0] = dd;
     out[1] = e;
     out[2] = f;
   }
 
   void finish() {
-    scale_inplace(Sigma, (int64_t)nts * ns * nk * nao2, 1.0 / nk, st);  // gw_cpu_kernel.cpp:55
+    const int64_t per_t = (int64_t)ns * nk * nao2;
+    if (nh == 2) {  // with the 1/nk of gw_cpu_kernel.cpp:55
+      unfold_sigma_kernel<<<grid_for(nts * per_t, 256), 256, 0, st>>>(acc, Sigma, nts, per_t, 1.0 / nk);
+      GB_CHECK_LAUNCH();
+    } else {
+      scale_inplace(Sigma, nts * per_t, 1.0 / nk, st);
+    }
     if (x2c) {
       const int64_t n = (int64_t)nts * 4 * nk * nao2;
       x2c_unpack_sigma_kernel<<<grid_for(n, 256), 256, 0, st>>>(Sigma, Sigma_out, nts, nk, (int)nao);
       GB_CHECK_LAUNCH();
     }
-    if (c.q0_on) apply_q0(c, G_in, Sigma_out, st);
+    if (c.q0_on) apply_q0(c, *wt, G_in, Sigma_out, st);
   }
 };
 

@@ -2,30 +2,27 @@
 // products on the 5th-generation tensor cores (tcgen05, kind::i8), FP64
 // recombination.
 //
-// Number format.  Every complex row of the left operand (and every complex
-// column of the right one) gets a power-of-two exponent e with max|Re|,|Im| <
-// 2^(e-1) over the contraction range (one bit of headroom).  Each real part is
-// rounded to X = rint(a 2^(7S-e)) and cut into S balanced base-128 digits,
-// a = 2^(e-7) (q_0 + q_1 2^-7 + ... + q_{S-1} 2^-7(S-1)) + r with q_s in [-64, 64]
-// (split_digits.cuh).  Products of slices s and t share the weight 2^-7(s+t); all
-// pairs with s + t = d accumulate into one INT32 accumulator "diagonal" d (pairs
-// with s + t >= S are dropped, the usual triangular Ozaki truncation).  Rounding
-// and balanced digits keep the representation error and the dropped products
-// zero-mean, so they do not add up in phase along the contraction.  The host
-// splits the contraction so that no diagonal can overflow INT32.
+// Number format.  Every complex row of the left operand (and every complex column of the right one) gets a
+// power-of-two exponent e with max|Re|,|Im| < 2^(e-1) over the contraction range.  Each real part is rounded to an
+// integer and cut into S balanced digits, a = 2^(e-7) (q_0 + q_1 B^-1 + ... + q_{S-1} B^-(S-1)) + r, base B = 256 for
+// up to six slices and 128 for seven and eight (split_digits.cuh).  Products of slices s and t share the weight
+// B^-(s+t); all pairs with s + t = d accumulate into one INT32 accumulator "diagonal" d (pairs with s + t >= S are
+// dropped, the usual triangular Ozaki truncation).  Rounding and balanced digits keep the representation error and the
+// dropped products zero-mean, so they do not add up in phase along the contraction.  The host splits the contraction
+// so that no diagonal can overflow INT32.
 //
-// Complex arithmetic.  A complex product becomes one real product through the
-// embedding  [Re A  -Im A; Im A  Re A] x [Re B; Im B]: the left operand is stored
-// with two interleaved real rows per complex row (2m: re,-im; 2m+1: im,re,
-// interleaved along K), the right operand as (re, im) pairs along K.  Real row
-// 2m of the result is Re C, row 2m+1 is Im C.
+// Complex arithmetic.  C = A B is computed as its transpose: the rows of the tensor-core tile are the columns n of B
+// (the large operand of every contraction), stored as (re, im) pairs along K, and its columns come from the rows m of
+// A in the real embedding, 2m: (re, -im) pairs and 2m+1: (im, re) pairs.  Columns 2m and 2m+1 of the result are then Re
+// and Im of C(m, n), in the same TMEM lane.  (With the embedding on the row side the two lie in different lanes, and
+// exchanging them took a fifth of the epilogue's instructions; the small operand's padding, 40 rows to 64, becomes
+// 80 columns of 80.)
 //
-// Tensor-core kernel.  One CTA computes 128 real rows x BN complex columns for
-// all S diagonals (S * BN <= 512 TMEM columns).  Warp 0 streams 64-byte K blocks
-// of every slice plane with TMA (64-byte swizzle) through a multi-stage mbarrier
-// ring, warp 1 issues the tcgen05.mma instructions from one thread, and 16
-// epilogue warps read the accumulators from TMEM (tcgen05.ld) and recombine in FP64.  Every
-// wait is bounded; on timeout the kernel records an error and returns.
+// Tensor-core kernel.  One CTA computes 128 values of n x BN / 2 values of m for all S diagonals (S * BN <= 512 TMEM
+// columns).  Warp 0 streams 64-byte K blocks of every slice plane with TMA (64-byte swizzle) through a multi-stage
+// mbarrier ring, warp 1 issues the tcgen05.mma instructions from one thread, warp 2 gathers the index maps and
+// exponents of the coming tile into shared memory, and 16 epilogue warps read the accumulators from TMEM (tcgen05.ld),
+// recombine in FP64 and store.  Every wait is bounded; on timeout the kernel records an error and returns.
 #include <cuda.h>
 #include <cudaTypedefs.h>
 
@@ -43,18 +40,16 @@ namespace gb200 {
 namespace {
 
 constexpr int KBLK = 64;          // bytes of K per pipeline stage (one 64B swizzle atom)
-constexpr int TILE_M = 128;       // real rows per CTA (64 complex rows)
-constexpr int SMEM_BUDGET = 216 * 1024;  // TMA ring + tables, under the 227 KB opt-in
+constexpr int TILE_R = 128;       // rows per CTA: complex columns n of the product
+constexpr int SMEM_MAX = 227 * 1024;  // the opt-in limit of a block
 constexpr int EPI_WARPS = 16;     // four per TMEM sub-partition: enough warps in flight to hide
                                   // the TMEM, FP64 and store latencies of the recombination
-constexpr int NWARPS = 2 + EPI_WARPS;  // producer, MMA, epilogue warps
-constexpr int EPI_THREADS = EPI_WARPS * 32;
-constexpr int EPI_CH = 32;                          // result columns per epilogue step
-constexpr int EPI_CG = EPI_CH / (EPI_WARPS / 4);  // columns of a step per epilogue warp
-static_assert(EPI_CG == 8, "epilogue column group: one tcgen05.ld of 8 columns");
+constexpr int EPI_FIRST = 3;      // producer, MMA and table warps before them
+constexpr int NWARPS = EPI_FIRST + EPI_WARPS;
+constexpr int EPI_CG = 8;         // result columns (4 complex) per TMEM read: one tcgen05.ld of 8 columns
 constexpr long long WAIT_LIMIT = 4000000000LL;  // clock64 cycles (~2 s)
 
-enum SplitErr { SERR_NONE = 0, SERR_TIMEOUT_PRODUCER = 1, SERR_TIMEOUT_MMA = 2, SERR_TIMEOUT_EPILOGUE = 3 };
+enum SplitErr { SERR_NONE = 0, SERR_TIMEOUT_PRODUCER = 1, SERR_TIMEOUT_MMA = 2, SERR_TIMEOUT_EPILOGUE = 3, SERR_TIMEOUT_TABLES = 4 };
 
 // ----------------------------------------------------------------------------
 // PTX wrappers
@@ -97,12 +92,23 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, volatil
   return true;
 }
 
-__device__ __forceinline__ void tma_load_2d(void* smem_dst, const CUtensorMap* map, int x, int y, uint64_t* bar) {
+__device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
           smem_u32(smem_dst)),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(smem_u32(bar))
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(smem_u32(bar))
       : "memory");
+}
+
+// one lane of a converged warp
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t is;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(is));
+  return is;
 }
 
 __device__ __forceinline__ void tmem_alloc(uint32_t* dst_smem, uint32_t ncols) {
@@ -114,17 +120,25 @@ __device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols));
 }
 
-__device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum) {
+// Issued by the one lane with `issue` set.  The whole warp runs the surrounding code, so that the operands, the same in
+// every lane, stay in uniform registers: computed by a single diverged thread they cost that thread several
+// instructions per operand, in competition with the epilogue warps of its scheduler.
+__device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accum,
+                                        uint32_t issue) {
   asm volatile(
-      "{\n\t.reg .pred p;\n\t"
+      "{\n\t.reg .pred p, q;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
-      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum));
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accum), "r"(issue));
 }
 
-__device__ __forceinline__ void umma_commit(uint64_t* bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
-               : "memory");
+__device__ __forceinline__ void umma_commit(uint64_t* bar, uint32_t issue) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\t"
+      "setp.ne.b32 q, %1, 0;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar)), "r"(issue)
+      : "memory");
 }
 
 __device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
@@ -135,8 +149,6 @@ __device__ __forceinline__ void tmem_ld8(uint32_t taddr, int32_t (&v)[8]) {
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                : "r"(taddr));
 }
-
-__device__ __forceinline__ void epi_bar() { asm volatile("bar.sync 1, %0;" ::"n"(EPI_THREADS) : "memory"); }
 
 __device__ __forceinline__ void tmem_wait_ld() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 
@@ -154,47 +166,34 @@ __device__ __forceinline__ uint64_t smem_desc_sw64(uint32_t saddr) {
 
 // Instruction descriptor: S32 accumulate, signed 8-bit A and B, both K-major, M=128, N=bn.
 __host__ __device__ constexpr uint32_t idesc_i8(int bn) {
-  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(TILE_M >> 4) << 24);
+  return (2u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(bn >> 3) << 17) | ((uint32_t)(TILE_R >> 4) << 24);
 }
 
 // ----------------------------------------------------------------------------
 // parameters
 // ----------------------------------------------------------------------------
-struct OperandSlices {
-  int64_t nrb = 1;             // reduced batch count
-  int dep[3] = {0, 0, 0};      // which batch components the operand depends on
-  int64_t R = 0;               // complex rows (A: M, B: N)
-  int64_t rows_pad = 0;        // real rows per plane
-  int64_t kpad = 0;            // bytes per row
-  int64_t e_ld = 0;            // exponents per reduced batch
-  int8_t* planes = nullptr;    // [nrb][S][rows_pad][kpad]
-  int32_t* expo = nullptr;     // [nrb][e_ld]
-};
-
 struct GemmParams {
   int S;
-  int BN;
+  int BN;         // tile columns: real columns of the embedded operand
   int stages;
-  int rows_fast;  // result rows are the unit-stride index (write-out walks rows first)
-  int nbuf;       // TMEM accumulator sets (2: epilogue overlaps the next tile's MMAs)
-  int tiles_m, tiles_n;
-  int nkb;
-  int ntiles_n;
-  int64_t M, N;
+  int tiles_r, tiles_c;
+  int nkb;        // K blocks of KBLK bytes
+  int nkk;        // K steps of 32 bytes
+  int overlap;    // launch-wide: two accumulator sets and resident row planes (short contractions)
+  int64_t M, N;   // complex rows of A (tile columns / 2) and columns of B (tile rows)
   int64_t nb0, nb1, nb2;
   int depA[3], depB[3];
-  int64_t rowsA_pad, rowsB_pad;
+  int64_t rowsA, rowsB;  // rows of a plane: 2 M and N
+  int ntile;       // tiles of this problem
   const int32_t* eA;
   const int32_t* eB;
   int64_t eA_ld, eB_ld;
   ZResult C;
   cplx alpha, beta;
   int alpha_pow2;  // alpha is real and a power of two (possibly negative)
-  int pair;        // the chunk is short enough that diagonal pairs (0,1), (2,3) fit int32 exactly
-  ExpoSink sink;   // exponents of a later contraction's operand, folded from the stored results
   int* err;
   // grouped launch: the problems' entries (tile ranges in order) and the total tile count; the
-  // launch-wide fields above (S, BN = the widest tile, stages, nbuf, err) size the shared ring
+  // launch-wide fields above (S, BN = the widest tile, stages, err) size the shared ring
   const struct GroupEntry* group;
   int ngroup;
   int64_t ntiles;
@@ -202,34 +201,10 @@ struct GemmParams {
 
 // one problem of a grouped launch: its tensor maps, parameters and first global tile
 struct alignas(64) GroupEntry {
-  CUtensorMap mA, mB;
+  CUtensorMap mR, mC;  // planes of the tile's rows (operand B) and columns (operand A)
   GemmParams p;
   int64_t tile_begin;
 };
-
-// a tile of the launch: its problem's parameters and maps, and its index within the problem
-struct TileRef {
-  const GemmParams* p;
-  const CUtensorMap* mA;
-  const CUtensorMap* mB;
-  int64_t t;
-};
-
-template <bool GROUPED>
-__device__ __forceinline__ TileRef tile_ref(const GemmParams& p, const CUtensorMap* mA, const CUtensorMap* mB, int64_t t) {
-  if constexpr (!GROUPED) {
-    return TileRef{&p, mA, mB, t};
-  } else {
-    int lo = 0, hi = p.ngroup - 1;  // last entry with tile_begin <= t
-    while (lo < hi) {
-      const int mid = (lo + hi + 1) / 2;
-      if (p.group[mid].tile_begin <= t) lo = mid;
-      else hi = mid - 1;
-    }
-    const GroupEntry& e = p.group[lo];
-    return TileRef{&e.p, &e.mA, &e.mB, t - e.tile_begin};
-  }
-}
 
 __device__ __forceinline__ int64_t reduced_batch(const int dep[3], int64_t b0, int64_t b1, int64_t b2, int64_t n1,
                                                  int64_t n2) {
@@ -251,10 +226,10 @@ struct SliceJob {
   int64_t R, K, k0;            // rows, K range [k0, k0 + K)
   int64_t n0, n1, n2;          // batch sizes of the GEMM
   int dep[3];
-  int embed;                   // 1: left operand (doubled rows), 0: right operand
+  int embed;                   // 1: operand A (doubled rows), 0: operand B
   int S;
-  int64_t rows_pad;            // real rows per plane
-  int64_t rpad;                // complex rows covered (rows_pad / 2 for the left operand)
+  int64_t rows_pad;            // real rows per plane (2 R for the embedded operand)
+  int64_t rpad;                // complex rows covered (R)
   int64_t kpad, e_ld;
   int8_t* out;
   int32_t* expo;
@@ -342,49 +317,66 @@ __global__ void __launch_bounds__(SL_NT, 4) slice_expo_kernel(SliceJob j) {
   }
 }
 
-// Ozaki digits of one real number: balanced base-128 digits of X = rint(a 2^(7S - e)), with one bit
-// of headroom in the row exponent e (split_digits.cuh).
+// base of the digits of S slices, and the power of two of the lowest diagonal's unit: a product of operands with
+// exponents ea, eb is 2^(ea + eb - unit_exp) times sum_d q_d B^(S-1-d)
+__host__ __device__ constexpr int digit_bits(int S) { return S <= 6 ? 8 : 7; }
+__host__ __device__ constexpr int unit_exp(int S) { return 14 + digit_bits(S) * (S - 1); }
 
-// Write the S digit planes of 8 consecutive K positions (from k) of row r with row exponent e,
-// including the zero padding of rows and K.  S is a compile-time constant, so every digit shift is
-// a constant and one plane's 16 bytes take four packed words (balanced_digit_word).
+// Write the S digit planes of 8 consecutive K positions (from k) of row r with row exponent e, including the zero
+// padding of K.  S is a compile-time constant, so every digit position is one, and a plane's 16 bytes take four
+// packed words.
 template <int S>
 __device__ __forceinline__ void write_digits(const SliceJob& j, const cplx (&vals)[8], int64_t rb, int64_t r, int64_t k,
                                              int e) {
   if (r >= j.rpad || 2 * k >= j.kpad) return;
-  // 2^(7S - e) in two exact power-of-two factors (the exponent can exceed the double range
-  // for rows of tiny magnitude)
-  const int ex = 7 * S - e;
-  const int ex1 = max(-1000, min(1000, ex));
-  const double sc1 = __longlong_as_double((long long)(ex1 + 1023) << 52);
-  const double sc2 = __longlong_as_double((long long)(max(-1022, min(1023, ex - ex1)) + 1023) << 52);
-  // X + bias of the rounded scaled values, (re, im) of the 8 positions in turn
+  constexpr bool WIDE = digit_bits(S) == 8;
+  // the scale 2^(8S - 1 - e) (base 128: 2^(7S - e)); as two exact factors where it leaves the double range
+  const int ex = (WIDE ? 8 * S - 1 : 7 * S) - e;
+  // the integers of the 8 positions, (re, im) in turn, plus the bias that makes their digits unsigned
   uint64_t u[16];
+  if (ex >= -1000 && ex <= 1000) {
+    const double sc = __longlong_as_double((long long)(ex + 1023) << 52);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    u[2 * i] = balanced_input((vals[i].x * sc1) * sc2, S);
-    u[2 * i + 1] = balanced_input((vals[i].y * sc1) * sc2, S);
+    for (int i = 0; i < 8; ++i) {
+      u[2 * i] = WIDE ? wide_input(vals[i].x * sc, S) : balanced_input(vals[i].x * sc, S);
+      u[2 * i + 1] = WIDE ? wide_input(vals[i].y * sc, S) : balanced_input(vals[i].y * sc, S);
+    }
+  } else {
+    const int ex1 = max(-1000, min(1000, ex));
+    const double sc1 = __longlong_as_double((long long)(ex1 + 1023) << 52);
+    const double sc2 = __longlong_as_double((long long)(max(-1022, min(1023, ex - ex1)) + 1023) << 52);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      u[2 * i] = WIDE ? wide_input((vals[i].x * sc1) * sc2, S) : balanced_input((vals[i].x * sc1) * sc2, S);
+      u[2 * i + 1] = WIDE ? wide_input((vals[i].y * sc1) * sc2, S) : balanced_input((vals[i].y * sc1) * sc2, S);
+    }
   }
   const int64_t plane = j.rows_pad * j.kpad;
-  int8_t* outb = j.out + rb * (int64_t)S * plane;
+  int8_t* outb = j.out + rb * (int64_t)S * plane + (j.embed ? 2 * r : r) * j.kpad + 2 * k;
 #pragma unroll
   for (int s = 0; s < S; ++s) {
     uint32_t w[4];  // bytes (re, im) of positions 2h and 2h + 1
 #pragma unroll
-    for (int h = 0; h < 4; ++h) w[h] = balanced_digit_word(u[4 * h], u[4 * h + 1], u[4 * h + 2], u[4 * h + 3], S, s);
+    for (int h = 0; h < 4; ++h)
+      w[h] = WIDE ? wide_digit_word(u[4 * h], u[4 * h + 1], u[4 * h + 2], u[4 * h + 3], S, s)
+                  : balanced_digit_word(u[4 * h], u[4 * h + 1], u[4 * h + 2], u[4 * h + 3], S, s);
     int8_t* p = outb + (int64_t)s * plane;
     if (j.embed) {
-      // row 2r: (re, -im) pairs; row 2r+1: (im, re) pairs
+      // row 2r: (re, -im) pairs; row 2r+1: (im, re) pairs.  (A base-256 digit of -128 has no negative: -im is cut into
+      // its own digits.)
       uint32_t w0[4], w1[4];
 #pragma unroll
       for (int h = 0; h < 4; ++h) {
-        w0[h] = __byte_perm(w[h], negate_bytes(w[h]), 0x7250);
+        const uint32_t neg = WIDE ? wide_digit_word(u[4 * h], wide_negate(u[4 * h + 1], S), u[4 * h + 2],
+                                                    wide_negate(u[4 * h + 3], S), S, s)
+                                  : __byte_perm(w[h], negate_bytes(w[h]), 0x7250);
+        w0[h] = neg;
         w1[h] = __byte_perm(w[h], 0u, 0x2301);
       }
-      *reinterpret_cast<uint4*>(p + (2 * r) * j.kpad + 2 * k) = make_uint4(w0[0], w0[1], w0[2], w0[3]);
-      *reinterpret_cast<uint4*>(p + (2 * r + 1) * j.kpad + 2 * k) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
+      *reinterpret_cast<uint4*>(p) = make_uint4(w0[0], w0[1], w0[2], w0[3]);
+      *reinterpret_cast<uint4*>(p + j.kpad) = make_uint4(w1[0], w1[1], w1[2], w1[3]);
     } else {
-      *reinterpret_cast<uint4*>(p + r * j.kpad + 2 * k) = make_uint4(w[0], w[1], w[2], w[3]);
+      *reinterpret_cast<uint4*>(p) = make_uint4(w[0], w[1], w[2], w[3]);
     }
   }
 }
@@ -530,143 +522,206 @@ __device__ __forceinline__ double int_to_double(int32_t x) {
   return __hiloint2double(0x43380000, (int)((uint32_t)x ^ 0x80000000u)) - 6755401588539392.0;
 }
 
-// Horner sum of the diagonals, sum_d q_d 128^(S-1-d), i.e. the value in units of
-// 2^(ea + eb - 7(S+1)).  With |q_d| < 2^31 the first four partial sums are exact (< 2^53), so
-// for S <= 5 the result is the exact sum rounded once.  The tensor-core epilogue evaluates the
-// same expression, so both engines agree bit for bit.
-__device__ __forceinline__ double combine_diagonals(const int32_t* q, int S) {
-  double v = int_to_double(q[0]);
-  for (int d = 1; d < S; ++d) v = fma(v, 128.0, int_to_double(q[d]));
-  return v;
-}
-
-// the factor of a result element: 2^ea (row) times 2^(eb - 7(S+1)) (column)
-__device__ __forceinline__ double result_scale(int ea, int eb, int S) { return pow2(ea) * pow2(eb - 7 * (S + 1)); }
-
-__device__ __forceinline__ void store_at(const GemmParams& p, cplx* dst, double re, double im, int ea, int eb) {
-  const double sc = result_scale(ea, eb, p.S);
-  cplx v = cmul(p.alpha, cmk(re * sc, im * sc));
-  if (p.beta.x != 0.0 || p.beta.y != 0.0) v = cadd(v, cmul(p.beta, *dst));
-  *dst = v;
-}
-
-__device__ __forceinline__ void store_result(const GemmParams& p, int64_t b0, int64_t b1, int64_t b2, int64_t m, int64_t n,
-                                             double re, double im, int ea, int eb) {
-  cplx* Cb = p.C.ptr + p.C.bat(b0, b1, b2);
-  store_at(p, Cb + p.C.row(m) + p.C.col(n), re, im, ea, eb);
-}
-
-// Horner sum of the S diagonals of W accumulator columns, as combine_diagonals.  With `pair`
-// (host check: |q_d| bounded by the chunk length) q_d 128 + q_(d+1) is exact in int32 for the
-// pairs (0,1) and (2,3), and the Horner sum over the pairs equals the one over single diagonals,
-// since every partial sum below 2^53 is exact.
-template <int S, int W>
-__device__ __forceinline__ void combine_cols(const int32_t (&q)[S][1][W], bool pair, double (&v)[W]) {
+// sum_d q_d B^(S-1-d) as a double, the value in units of 2^(ea + eb - unit_exp).  Up to five slices the sum is formed
+// exactly in 64-bit integers (|q_d| < 2^31, so it is below 2^63) and rounded once: four multiply-adds and three FP64
+// operations where a Horner sum over converted diagonals takes fourteen.  Both engines use this function, so they agree
+// bit for bit.
+template <int S>
+__device__ __forceinline__ double combine_diagonals(const int32_t (&q)[S]) {
   if constexpr (S <= 5) {
-    if (pair) {
+    long long t = q[S - 1];
 #pragma unroll
-      for (int j = 0; j < W; ++j) {
-        double a = int_to_double(q[0][0][j] * 128 + q[1][0][j]);
-        if constexpr (S >= 4) a = fma(a, 16384.0, int_to_double(q[2][0][j] * 128 + q[3][0][j]));
-        if constexpr (S == 3) a = fma(a, 128.0, int_to_double(q[2][0][j]));
-        if constexpr (S == 5) a = fma(a, 128.0, int_to_double(q[4][0][j]));
-        v[j] = a;
-      }
-      return;
-    }
-  }
+    for (int i = 1; i < (S < 4 ? S : 4); ++i) t += (long long)q[S - 1 - i] * (1 << (8 * i));
+    int hi = (int)(t >> 32);
+    if constexpr (S == 5) hi += q[0];
+    const double lo = __hiloint2double(0x43300000, (int)(uint32_t)t) - 4503599627370496.0;  // the low word, unsigned
+    return fma(int_to_double(hi), 4294967296.0, lo);
+  } else {
+    constexpr double B = digit_bits(S) == 8 ? 256.0 : 128.0;
+    double v = int_to_double(q[0]);
 #pragma unroll
-  for (int j = 0; j < W; ++j) {
-    double a = 0.0;
-#pragma unroll
-    for (int d = 0; d < S; ++d) a = fma(a, 128.0, int_to_double(q[d][0][j]));
-    v[j] = a;
+    for (int d = 1; d < S; ++d) v = fma(v, B, int_to_double(q[d]));
+    return v;
   }
 }
 
 // ----------------------------------------------------------------------------
 // tcgen05 core
 // ----------------------------------------------------------------------------
+// Short contractions (over up to RES_KB K blocks: 64 orbitals) run in overlap mode: two accumulator sets of half the
+// width, so that the epilogue of a tile runs beside the MMAs of the next, and the row planes of a tile kept in shared
+// memory (two sets) for the column tiles that share them, which halves what a tile reads from L2.
+constexpr int RES_KB = 2;
+constexpr int OVERLAP_MAX_S = 5;  // (six slices leave no room for two sets of rows)
+
 struct SmemLayout {
-  int stage_bytes, a_plane_bytes, b_plane_bytes, stages, ring_bytes, ctile_bytes;
+  int r_plane_bytes;  // one row plane of a K block
+  int rows_bytes;     // resident row planes, [2][S][RES_KB] (0: they are part of the stages)
+  int stage_rows;     // row-plane bytes of a stage
+  int stage_bytes, stages, ring_bytes;
 };
 
-__host__ __device__ inline SmemLayout smem_layout(int S, int BN, int stages) {
+__host__ __device__ inline SmemLayout smem_layout(int S, int BN, int stages, int overlap) {
   SmemLayout L;
-  L.a_plane_bytes = TILE_M * KBLK;
-  L.b_plane_bytes = BN * KBLK;
-  L.stage_bytes = S * (L.a_plane_bytes + L.b_plane_bytes);
+  L.r_plane_bytes = TILE_R * KBLK;
+  L.rows_bytes = overlap ? 2 * S * RES_KB * L.r_plane_bytes : 0;
+  L.stage_rows = overlap ? 0 : S * L.r_plane_bytes;
+  L.stage_bytes = L.stage_rows + S * BN * KBLK;
   L.stages = stages;
-  L.ring_bytes = stages * L.stage_bytes;
-  L.ctile_bytes = 0;  // the epilogue stores from registers (no staging tile)
+  L.ring_bytes = L.rows_bytes + stages * L.stage_bytes;
   return L;
 }
 
-// one set of per-tile epilogue tables: row and column offsets of C, column factors, row exponents
-// and the exponent-sink entries of the column groups (BN / 8 of the BN 4-byte slots at the end)
-__host__ __device__ inline int table_set_bytes(int BN) {
-  return ((TILE_M / 2) * 8 + BN * 16 + (TILE_M / 2 + BN) * 4 + 15) / 16 * 16;
-}
-
-// bytes after the tile ring: barriers, TMEM slot, flags, two sets of per-tile tables
-__host__ __device__ inline int misc_bytes(int stages, int BN) {
-  return (2 * stages + 4) * 8 + 32 + 2 * table_set_bytes(BN) + 64;
-}
-
-struct TileCoord {
-  int64_t b0, b1, b2, rbA, rbB, mrow0, ncol0;
+// What the epilogue needs of a tile: this head, then per complex column its offset in C and factor 2^(eA - unit_exp);
+// and, in one of two sets that consecutive tiles on the same rows share, per row its offset and factor 2^eB (alpha).
+struct TileHead {
+  cplx* C;
+  int rlim, clim;  // rows and complex columns inside the result
+  int ngroups;     // groups of EPI_CG columns
+  int bn;
+  int scaled;      // alpha is not in the factors
+  int has_beta;
+  int rowset;
+  int pad[3];
+  cplx alpha, beta;
 };
+static_assert(sizeof(TileHead) % 16 == 0, "tables follow the head");
 
-__device__ __forceinline__ TileCoord tile_coord(const GemmParams& p, int64_t t) {
-  // tile and batch counts fit 32 bits (the host checks), so the divisions are 32-bit
-  TileCoord c;
-  const uint32_t per_batch = (uint32_t)p.tiles_m * (uint32_t)p.tiles_n;
-  const uint32_t t32 = (uint32_t)t;
-  const uint32_t bz = t32 / per_batch;
-  const uint32_t rem = t32 - bz * per_batch;
-  const uint32_t by = rem / (uint32_t)p.tiles_n, bx = rem - by * (uint32_t)p.tiles_n;  // N fastest: neighbours share A
-  const uint32_t nb2 = (uint32_t)p.nb2, nb1 = (uint32_t)p.nb1;
-  const uint32_t bq = bz / nb2;
-  c.b2 = bz - bq * nb2;
-  c.b1 = bq % nb1;
-  c.b0 = bq / nb1;
-  c.rbA = reduced_batch(p.depA, c.b0, c.b1, c.b2, p.nb1, p.nb2);
-  c.rbB = reduced_batch(p.depB, c.b0, c.b1, c.b2, p.nb1, p.nb2);
-  c.mrow0 = (int64_t)by * TILE_M;
-  c.ncol0 = (int64_t)bx * p.BN;
-  return c;
+constexpr int ROW_TABLE_BYTES = TILE_R * 16;
+__host__ __device__ inline int table_set_bytes(int BN) { return (int)sizeof(TileHead) + BN / 2 * 16; }
+
+// bytes after the tile ring: barriers, TMEM slot, flags, two sets of row and of per-tile tables
+__host__ __device__ inline int misc_bytes(int stages, int BN) {
+  return (2 * stages + 12) * 8 + 32 + 2 * (ROW_TABLE_BYTES + table_set_bytes(BN)) + 64;
 }
+
+// A CTA's walk over its tiles: its problem's parameters and maps, and the tile's position as digits (column tile, row
+// tile, batch; columns fastest, so neighbours share rows), advanced by adding the digits of the step.  Tile and batch
+// counts fit 32 bits (the host checks).
+template <bool GROUPED>
+struct TileWalk {
+  const GemmParams* launch;
+  const GemmParams* q;
+  const CUtensorMap* mR;
+  const CUtensorMap* mC;
+  uint32_t t, t_end, step;  // tile of the launch
+  uint32_t local;           // tile of the problem
+  uint32_t bx, by, bz, sx, sy, sz;
+  uint32_t b0, b1, b2, rbA, rbB;
+  bool new_rows;            // other rows than the tile before (always so at the start of a run of column tiles)
+
+  __device__ __forceinline__ void batch() {
+    const uint32_t nb2 = (uint32_t)q->nb2, nb1 = (uint32_t)q->nb1;
+    const uint32_t bq = nb2 == 1 ? bz : bz / nb2;
+    b2 = bz - bq * nb2;
+    b0 = nb1 == 1 ? bq : bq / nb1;
+    b1 = bq - b0 * nb1;
+    rbA = (uint32_t)reduced_batch(q->depA, b0, b1, b2, nb1, nb2);
+    rbB = (uint32_t)reduced_batch(q->depB, b0, b1, b2, nb1, nb2);
+  }
+  __device__ __forceinline__ void locate() {
+    if constexpr (GROUPED) {
+      int lo = 0, hi = launch->ngroup - 1;  // last entry with tile_begin <= t
+      while (lo < hi) {
+        const int mid = (lo + hi + 1) / 2;
+        if (launch->group[mid].tile_begin <= (int64_t)t) lo = mid;
+        else hi = mid - 1;
+      }
+      const GroupEntry& e = launch->group[lo];
+      q = &e.p;
+      mR = &e.mR;
+      mC = &e.mC;
+      local = t - (uint32_t)e.tile_begin;
+    } else {
+      local = t;
+    }
+    const uint32_t tc = (uint32_t)q->tiles_c, tr = (uint32_t)q->tiles_r;
+    uint32_t x = local / tc;
+    bx = local - x * tc;
+    bz = x / tr;
+    by = x - bz * tr;
+    x = step / tc;
+    sx = step - x * tc;
+    sz = x / tr;
+    sy = x - sz * tr;
+    batch();
+    new_rows = true;
+  }
+  __device__ __forceinline__ TileWalk(const GemmParams& p, const CUtensorMap* r, const CUtensorMap* c, uint32_t first,
+                                      uint32_t end, uint32_t st)
+      : launch(&p), q(&p), mR(r), mC(c), t(first), t_end(end), step(st) {
+    if (t < t_end) locate();
+  }
+  __device__ __forceinline__ bool more() const { return t < t_end; }
+  __device__ __forceinline__ void next() {
+    t += step;
+    if (t >= t_end) return;
+    local += step;
+    if (GROUPED && local >= (uint32_t)q->ntile) {
+      locate();
+      return;
+    }
+    const uint32_t tc = (uint32_t)q->tiles_c, tr = (uint32_t)q->tiles_r, oy = by;
+    bx += sx;
+    by += sy;
+    if (bx >= tc) {
+      bx -= tc;
+      ++by;
+    }
+    uint32_t dz = sz;
+    if (by >= tr) {
+      by -= tr;
+      ++dz;
+    }
+    new_rows = by != oy || dz != 0;
+    if (dz) {
+      bz += dz;
+      batch();
+    }
+  }
+  __device__ __forceinline__ int row0() const { return (int)by * TILE_R; }
+  __device__ __forceinline__ int col0() const { return (int)bx * q->BN; }
+};
 
 // Persistent tensor-core kernel: every CTA walks tiles blockIdx.x, +gridDim.x, ...
 //  warp 0       TMA producer (one thread), a ring of `stages` K blocks that runs across tiles
-//  warp 1       MMA issuer (one thread), `nbuf` TMEM accumulator sets of S * BN columns
-//  warps 2..    epilogue (EPI_WARPS): TMEM -> registers -> FP64 recombination -> stores to C
-// With nbuf = 2 the epilogue of one tile overlaps the MMAs of the next.
-template <int SS, bool GROUPED, bool SINK>
+//  warp 1       MMA issuer (one thread), one TMEM accumulator set of S * BN columns
+//  warp 2       tables: what the epilogue needs of the next tile, in two alternating sets
+//  warps 3..    epilogue (EPI_WARPS): TMEM -> registers -> FP64 recombination -> stores to C
+// Bound by the MMAs for long contractions (8192 multiply-adds a cycle and SM) and by the instructions of the epilogue
+// for the short ones (K = 40: 3 K steps of 720 cycles a tile against 12 column groups per scheduler), which is why the
+// tile's index arithmetic has a warp of its own and no block barrier separates tiles.
+template <int SS, bool GROUPED>
 __global__ void __launch_bounds__(NWARPS * 32, 1)
-    split_gemm_tc_kernel(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, GemmParams p) {
+    split_gemm_tc_kernel(const __grid_constant__ CUtensorMap mapR, const __grid_constant__ CUtensorMap mapC,
+                         const __grid_constant__ GemmParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-  const SmemLayout L = smem_layout(p.S, p.BN, p.stages);
-  uint8_t* tiles = smem;
-  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L.ring_bytes + L.ctile_bytes);
+  const SmemLayout L = smem_layout(p.S, p.BN, p.stages, p.overlap);
+  uint8_t* rows_smem = smem;
+  uint8_t* tiles = smem + L.rows_bytes;
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + L.ring_bytes);
   uint64_t* empty_bar = full_bar + L.stages;
-  uint64_t* accf_bar = empty_bar + L.stages;   // [2]
-  uint64_t* acce_bar = accf_bar + 2;           // [2]
-  uint8_t* misc = reinterpret_cast<uint8_t*>(acce_bar + 2);
+  uint64_t* accf_bar = empty_bar + L.stages;   // [2] accumulator set complete
+  uint64_t* acce_bar = accf_bar + 2;           // [2] accumulator set read
+  uint64_t* tabf_bar = acce_bar + 2;           // [2] table set filled
+  uint64_t* tabe_bar = tabf_bar + 2;           // [2] table set read
+  uint64_t* rowf_bar = tabe_bar + 2;           // [2] resident rows loaded
+  uint64_t* rowe_bar = rowf_bar + 2;           // [2] resident rows no longer read
+  uint8_t* misc = reinterpret_cast<uint8_t*>(rowe_bar + 2);
   uint32_t* tmem_base_slot = reinterpret_cast<uint32_t*>(misc);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(misc + 4);
-  volatile int* epi_ok = reinterpret_cast<volatile int*>(misc + 8);  // [2], per tile parity
-  uint8_t* tables = misc + 32;                                          // [2] table sets
+  uint8_t* row_tables = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(misc + 8) + 15) & ~uintptr_t(15));
+  uint8_t* tables = row_tables + 2 * ROW_TABLE_BYTES;
   const int tsb = table_set_bytes(p.BN);
 
   const int warp = threadIdx.x / 32, lane = threadIdx.x % 32;
   constexpr int S = SS;
-  const int nbuf = p.nbuf;
+  const int nbuf = p.overlap ? 2 : 1;
   const uint32_t acc_cols = (uint32_t)(S * p.BN);
   const uint32_t need = acc_cols * (uint32_t)nbuf;
   const uint32_t ncols_alloc = need <= 32 ? 32 : need <= 64 ? 64 : need <= 128 ? 128 : need <= 256 ? 256 : 512;
-  const int64_t ntiles = GROUPED ? p.ntiles : (int64_t)p.tiles_m * p.tiles_n * p.nb0 * p.nb1 * p.nb2;
+  const int64_t ntiles = GROUPED ? p.ntiles : (int64_t)p.tiles_r * p.tiles_c * p.nb0 * p.nb1 * p.nb2;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < L.stages; ++s) {
@@ -674,11 +729,14 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
       mbar_init(&empty_bar[s], 1);
     }
     for (int b = 0; b < 2; ++b) {
+      mbar_init(&rowf_bar[b], 1);
+      mbar_init(&rowe_bar[b], 1);
       mbar_init(&accf_bar[b], 1);
       mbar_init(&acce_bar[b], EPI_WARPS);  // every epilogue warp releases the set it has read
+      mbar_init(&tabf_bar[b], 1);
+      mbar_init(&tabe_bar[b], EPI_WARPS);
     }
     *abort_flag = 0;
-    epi_ok[0] = epi_ok[1] = 1;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
@@ -688,251 +746,303 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
   tc_fence_after();
   const uint32_t tmem_base = *tmem_base_slot;
 
-  int64_t issued = 0;  // producer: K blocks issued in total
+  // this CTA's tiles: every gridDim.x-th one, or, in overlap mode, a contiguous range (columns fastest), in which
+  // most neighbours share their rows
+  const uint32_t t_first = p.overlap ? (uint32_t)(ntiles * blockIdx.x / gridDim.x) : blockIdx.x;
+  const uint32_t t_end = p.overlap ? (uint32_t)(ntiles * (blockIdx.x + 1) / gridDim.x) : (uint32_t)ntiles;
+  const uint32_t t_step = p.overlap ? 1u : gridDim.x;
+  const int nstage = L.stages;
+
+  uint32_t issued = 0;  // producer: K blocks issued in total
+  uint32_t nrows = 0;   // producer: row tiles loaded (overlap mode)
   if (warp == 0) {
     if (lane == 0) {
-      int64_t it = 0;
+      int st = 0;
+      uint32_t ph = 1;  // a fresh barrier's previous phase counts as complete
       const GemmParams* last_q = nullptr;
-      for (int64_t t = blockIdx.x; t < ntiles && !*abort_flag; t += gridDim.x) {
-        const TileRef tr = tile_ref<GROUPED>(p, &mapA, &mapB, t);
-        const GemmParams& q = *tr.p;
+      for (TileWalk<GROUPED> w(p, &mapR, &mapC, t_first, t_end, t_step); w.more() && !*abort_flag; w.next()) {
+        const GemmParams& q = *w.q;
         if constexpr (GROUPED) {
-          if (tr.p != last_q) {
+          if (w.q != last_q) {
             // the problem's tensor maps live in global memory that the host rewrites between
             // launches: order those writes before the tensor-map reads of the loads
-            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tr.mA) : "memory");
-            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(tr.mB) : "memory");
-            last_q = tr.p;
+            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(w.mR) : "memory");
+            asm volatile("fence.proxy.tensormap::generic.acquire.gpu [%0], 128;" ::"l"(w.mC) : "memory");
+            last_q = w.q;
           }
         }
-        const TileCoord tc = tile_coord(q, tr.t);
-        const int bpb = q.BN * KBLK;  // bytes of one B plane of this tile
-        const uint32_t tile_stage_bytes = (uint32_t)(S * (L.a_plane_bytes + bpb));
-        const int nkb = q.nkb;
-        const int64_t rowsA_pad = q.rowsA_pad, rowsB_pad = q.rowsB_pad;
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int st = (int)(it % L.stages);
-          const uint32_t ph = (uint32_t)((it / L.stages) & 1);
-          if (it >= L.stages && !mbar_wait(&empty_bar[st], ph ^ 1, abort_flag)) {
+        // all S planes of a K block in one load each; rows past a plane's end come as zeros
+        const uint32_t rbytes = (uint32_t)(S * L.r_plane_bytes);
+        const uint32_t tile_stage_bytes = (uint32_t)(S * q.BN * KBLK) + (p.overlap ? 0u : rbytes);
+        const int nkb = q.nkb, row0 = w.row0(), col0 = w.col0(), zr = (int)w.rbB * S, zc = (int)w.rbA * S;
+        if (p.overlap && w.new_rows) {
+          const uint32_t rset = nrows & 1;
+          if (!mbar_wait(&rowe_bar[rset], ((nrows >> 1) & 1) ^ 1, abort_flag)) {
             atomicExch(p.err, SERR_TIMEOUT_PRODUCER);
             *abort_flag = 1;
             break;
           }
+          ++nrows;
+          mbar_expect_tx(&rowf_bar[rset], rbytes * (uint32_t)nkb);
+          for (int kb = 0; kb < nkb; ++kb)
+            tma_load_3d(rows_smem + (size_t)(rset * RES_KB + kb) * rbytes, w.mR, kb * KBLK, row0, zr, &rowf_bar[rset]);
+        }
+        bool ok = true;
+        for (int kb = 0; kb < nkb; ++kb) {
+          if (!mbar_wait(&empty_bar[st], ph, abort_flag)) {
+            ok = false;
+            break;
+          }
           uint8_t* sbase = tiles + (size_t)st * L.stage_bytes;
           mbar_expect_tx(&full_bar[st], tile_stage_bytes);
-          for (int s = 0; s < S; ++s) {
-            const int ya = (int)((tc.rbA * S + s) * rowsA_pad + tc.mrow0);
-            tma_load_2d(sbase + s * L.a_plane_bytes, tr.mA, kb * KBLK, ya, &full_bar[st]);
+          if (!p.overlap) tma_load_3d(sbase, w.mR, kb * KBLK, row0, zr, &full_bar[st]);
+          tma_load_3d(sbase + L.stage_rows, w.mC, kb * KBLK, col0, zc, &full_bar[st]);
+          ++issued;
+          if (++st == nstage) {
+            st = 0;
+            ph ^= 1;
           }
-          uint8_t* bbase = sbase + S * L.a_plane_bytes;
-          for (int u = 0; u < S; ++u) {
-            const int yb = (int)((tc.rbB * S + u) * rowsB_pad + tc.ncol0);
-            tma_load_2d(bbase + u * bpb, tr.mB, kb * KBLK, yb, &full_bar[st]);
-          }
-          issued = it + 1;
+        }
+        if (!ok) {
+          atomicExch(p.err, SERR_TIMEOUT_PRODUCER);
+          *abort_flag = 1;
+          break;
         }
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
-      int64_t it = 0, tcount = 0;
-      // Slice plane s of A meets the S - s first planes of B at once: they lie one after another in the stage, and
-      // their products belong to the consecutive diagonals s .. S - 1, so they are one MMA of (S - s) BN columns (two
-      // when that is above 256).  For S = 5 and 96 columns a 32-byte K step is 8 MMAs that run at the tensor pipe's
-      // 8192 multiply-adds a cycle; one MMA per pair of planes (15 of 96 columns) is bound by the shared-memory reads
-      // of its operands (56 cycles for 48 of work) and by the issuing thread's descriptor arithmetic.
-      // The descriptors' upper halves and the widths are fixed per tile; per stage only base addresses are added.
-      const uint32_t desc_hi = (uint32_t)(smem_desc_sw64(0) >> 32);
-      const uint32_t ring_lo = (uint32_t)smem_desc_sw64(smem_u32(tiles));
-      const uint32_t stage_lo = (uint32_t)L.stage_bytes >> 4, plane_lo = (uint32_t)L.a_plane_bytes >> 4;
-      uint32_t id0[S], id1[S], dcol1[S], boff1[S];  // per A plane: instruction descriptors of the two parts, and the
-                                                    // second part's column and B row offsets (id1 = 0: one part)
-      int last_bn = 0;
-      for (int64_t t = blockIdx.x; t < ntiles && !*abort_flag; t += gridDim.x, ++tcount) {
-        const TileRef tr = tile_ref<GROUPED>(p, &mapA, &mapB, t);
-        const int tbn = tr.p->BN, nkb = tr.p->nkb;
-        if (tbn != last_bn) {
-          last_bn = tbn;
-#pragma unroll
-          for (int s = 0; s < S; ++s) {
-            const int n = (S - s) * tbn;
-            const int n0 = n <= 256 ? n : (n / 2 + 15) / 16 * 16;
-            id0[s] = idesc_i8(n0);
-            id1[s] = n > n0 ? idesc_i8(n - n0) : 0u;
-            dcol1[s] = (uint32_t)n0;
-            boff1[s] = (uint32_t)(n0 * KBLK) >> 4;
-          }
-        }
-        const int buf = (int)(tcount % nbuf);
-        const int64_t use = tcount / nbuf;
-        if (use > 0 && !mbar_wait(&acce_bar[buf], (uint32_t)((use - 1) & 1), abort_flag)) {
-          atomicExch(p.err, SERR_TIMEOUT_MMA);
-          *abort_flag = 1;
-          break;
-        }
+    // Slice plane s of the rows meets the S - s first planes of the columns at once: they lie one after another in the
+    // stage, and their products belong to the consecutive diagonals s .. S - 1, so they are one MMA of (S - s) BN
+    // columns (two when that is above 256).  For S = 5 and 96 columns a 32-byte K step is 8 MMAs that run at the tensor
+    // pipe's 8192 multiply-adds a cycle; one MMA per pair of planes (15 of 96 columns) is bound by the shared-memory
+    // reads of its operands (56 cycles for 48 of work).  The descriptors' upper halves and the widths are fixed per
+    // tile; per stage only base addresses are added.
+    const uint32_t issue = elect_one();
+    const uint32_t desc_hi = (uint32_t)(smem_desc_sw64(0) >> 32);
+    const uint32_t ring_lo = (uint32_t)smem_desc_sw64(smem_u32(tiles));
+    const uint32_t rows_lo = (uint32_t)smem_desc_sw64(smem_u32(rows_smem));
+    const uint32_t stage_lo = (uint32_t)L.stage_bytes >> 4, plane_lo = (uint32_t)L.r_plane_bytes >> 4;
+    const uint32_t cols_lo = (uint32_t)L.stage_rows >> 4;
+    const int overlap = p.overlap;
+    int st = 0, buf = 0;
+    uint32_t ph = 0, acc_ph = 1, rows_seen = 0;
+    for (TileWalk<GROUPED> w(p, &mapR, &mapC, t_first, t_end, t_step); w.more(); w.next()) {
+      if (__any_sync(0xffffffffu, *abort_flag)) break;
+      const int tbn = w.q->BN, nkb = w.q->nkb;
+      int ksteps = w.q->nkk;  // 32-byte K steps left
+      bool ok = mbar_wait(&acce_bar[buf], acc_ph, abort_flag);
+      if (overlap && w.new_rows) {
+        if (rows_seen > 0) umma_commit(&rowe_bar[(rows_seen - 1) & 1], issue);  // the previous rows' MMAs are all issued
+        ok = ok && mbar_wait(&rowf_bar[rows_seen & 1], (rows_seen >> 1) & 1, abort_flag);
+        ++rows_seen;
+      }
+      const uint32_t acc = tmem_base + (uint32_t)buf * acc_cols;
+      const uint32_t rows_set = rows_lo + ((rows_seen - 1) & 1) * (uint32_t)(RES_KB * S) * plane_lo;
+      uint32_t accum = 0;
+      for (int kb = 0; kb < nkb; ++kb) {
+        ok = ok && mbar_wait(&full_bar[st], ph, abort_flag);
+        if (!__all_sync(0xffffffffu, ok)) break;
         tc_fence_after();
-        const uint32_t acc = tmem_base + (uint32_t)buf * acc_cols;
-        bool ok = true;
-        for (int kb = 0; kb < nkb; ++kb, ++it) {
-          const int st = (int)(it % L.stages);
-          const uint32_t ph = (uint32_t)((it / L.stages) & 1);
-          if (!mbar_wait(&full_bar[st], ph, abort_flag)) {
-            atomicExch(p.err, SERR_TIMEOUT_MMA);
-            *abort_flag = 1;
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t a_lo = ring_lo + (uint32_t)st * stage_lo, b_lo = a_lo + (uint32_t)S * plane_lo;
+        const uint32_t s_lo = ring_lo + (uint32_t)st * stage_lo;
+        const uint32_t a_lo = overlap ? rows_set + (uint32_t)(kb * S) * plane_lo : s_lo;  // row planes of this K block
+        const uint32_t b_lo = s_lo + cols_lo;
 #pragma unroll
-          for (int kk = 0; kk < KBLK / 32; ++kk) {
+        for (int kk = 0; kk < KBLK / 32; ++kk) {
+          if (kk < ksteps) {
             const uint64_t bd = ((uint64_t)desc_hi << 32) | (b_lo + 2 * kk);
 #pragma unroll
             for (int s = 0; s < S; ++s) {
               const uint64_t ad = ((uint64_t)desc_hi << 32) | (a_lo + (uint32_t)s * plane_lo + 2 * kk);
               const uint32_t dt = acc + (uint32_t)(s * tbn);
-              const uint32_t accum = (kb > 0 || kk > 0 || s > 0) ? 1u : 0u;
-              umma_i8(dt, ad, bd, id0[s], accum);
-              if (id1[s]) umma_i8(dt + dcol1[s], ad, bd + boff1[s], id1[s], accum);
+              const int n = (S - s) * tbn;
+              if (n <= 256) {
+                umma_i8(dt, ad, bd, idesc_i8(n), accum, issue);
+              } else {
+                const int n0 = (n / 2 + 15) / 16 * 16;
+                umma_i8(dt, ad, bd, idesc_i8(n0), accum, issue);
+                umma_i8(dt + (uint32_t)n0, ad, bd + (uint32_t)(n0 * (KBLK / 16)), idesc_i8(n - n0), accum, issue);
+              }
+              accum = 1;
             }
           }
-          umma_commit(&empty_bar[st]);
         }
-        if (!ok) break;
-        umma_commit(&accf_bar[buf]);
+        ksteps -= KBLK / 32;
+        umma_commit(&empty_bar[st], issue);
+        if (++st == nstage) {
+          st = 0;
+          ph ^= 1;
+        }
+      }
+      if (!__all_sync(0xffffffffu, ok)) {
+        if (lane == 0) {
+          atomicExch(p.err, SERR_TIMEOUT_MMA);
+          *abort_flag = 1;
+        }
+        break;
+      }
+      umma_commit(&accf_bar[buf], issue);
+      if (++buf == nbuf) {
+        buf = 0;
+        acc_ph ^= 1;
       }
     }
-  } else {
-    // epilogue warps: TMEM sub-partition = warp % 4; the EPI_WARPS / 4 warps of a sub-partition
-    // take consecutive EPI_CG-column groups of each step.  Lanes 2j and 2j+1 hold the real and
-    // imaginary row of one complex result row; one shuffle gives each lane both parts of half of
-    // its columns, which it stores straight to C.  The tables of consecutive tiles alternate
-    // between two sets, so one named barrier per tile separates their writes from their reads.
-    const int sp = warp % 4;
-    const int grp = (warp - 2) / 4;
-    const int row = sp * 32 + lane;  // real row inside the tile
-    const int et = threadIdx.x - 64;  // 0..EPI_THREADS-1
-    const int mloc = row / 2;
-    const int r = row & 1;
-    constexpr int H = EPI_CG / 2;
-    int64_t tcount = 0;
-    for (int64_t t = blockIdx.x; t < ntiles; t += gridDim.x, ++tcount) {
-      const TileRef tr = tile_ref<GROUPED>(p, &mapA, &mapB, t);
-      const GemmParams& q = *tr.p;  // this tile's problem
-      const TileCoord tc = tile_coord(q, tr.t);
-      const int buf = (int)(tcount % nbuf);
-      const int64_t use = tcount / nbuf;
-      uint8_t* tb = tables + (tcount & 1) * tsb;
-      int64_t* sh_rowC = reinterpret_cast<int64_t*>(tb);
-      int64_t* sh_colC = sh_rowC + TILE_M / 2;
-      double* sh_csc = reinterpret_cast<double*>(sh_colC + q.BN);  // column factors 2^(eb - 7(S+1))
-      int32_t* sh_eA = reinterpret_cast<int32_t*>(sh_csc + q.BN);
-      int32_t* sh_key = sh_eA + TILE_M / 2;  // exponent-sink entry per group of 8 columns
-      // (filled while the MMAs of this tile run)
-      const int ntab = TILE_M / 2 + q.BN + ((SINK && q.sink.expo) ? q.BN / EPI_CG : 0);
-      for (int i = et; i < ntab; i += EPI_THREADS) {
-        if (i >= TILE_M / 2 + q.BN) {
-          const int64_t n = tc.ncol0 + (int64_t)(i - TILE_M / 2 - q.BN) * EPI_CG;
-          const ExpoSink& sk = q.sink;
-          sh_key[i - TILE_M / 2 - q.BN] = (int32_t)(sk.c0 * tc.b0 + sk.c1 * tc.b1 + sk.c2 * tc.b2 +
-                                                    ((n / sk.d1) % sk.m1) * sk.s1 + (n / sk.d2) * sk.s2);
-        } else if (i < TILE_M / 2) {
-          const int64_t m = tc.mrow0 / 2 + i;
-          sh_eA[i] = m < q.M ? q.eA[tc.rbA * q.eA_ld + m] : 0;
-          sh_rowC[i] = m < q.M ? q.C.row(m) : 0;
-        } else {
-          const int64_t n = tc.ncol0 + (i - TILE_M / 2);
-          const int eb = n < q.N ? q.eB[tc.rbB * q.eB_ld + n] : 0;
-          sh_colC[i - TILE_M / 2] = n < q.N ? q.C.col(n) : 0;
-          sh_csc[i - TILE_M / 2] = pow2(eb - 7 * (S + 1));
+  } else if (warp == 2) {
+    uint32_t tcount = 0, nr = 0;  // tiles, row tables written (the last in set (nr - 1) & 1)
+    for (TileWalk<GROUPED> w(p, &mapR, &mapC, t_first, t_end, t_step); w.more(); w.next(), ++tcount) {
+      const int set = (int)(tcount & 1);
+      const GemmParams& q = *w.q;
+      const int64_t row0 = w.row0(), m0 = w.col0() / 2;
+      const int64_t rlim = q.N - row0, clim = q.M - m0;
+      // this tile's exponents are on their way while the table set is waited for
+      const int32_t* eA = q.eA + w.rbA * q.eA_ld + m0;
+      const bool cin = lane < clim && lane < q.BN / 2;
+      const int e0 = cin ? eA[lane] : 0;
+      const int64_t o0 = cin ? q.C.row(m0 + lane) : 0;
+      bool ok = true;
+      if (lane == 0) ok = mbar_wait(&tabe_bar[set], ((tcount >> 1) & 1) ^ 1, abort_flag);
+      if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) {
+        if (lane == 0) {
+          atomicExch(p.err, SERR_TIMEOUT_TABLES);
+          *abort_flag = 1;
+        }
+        break;
+      }
+      uint8_t* tb = tables + set * tsb;
+      int64_t* coff = reinterpret_cast<int64_t*>(tb + sizeof(TileHead));
+      double* csc = reinterpret_cast<double*>(coff + q.BN / 2);
+      if (w.new_rows) {
+        // new rows go to the other row set; its last tile lies at least two tiles back and has been stored
+        int64_t* roff = reinterpret_cast<int64_t*>(row_tables + (nr & 1) * ROW_TABLE_BYTES);
+        double* rsc = reinterpret_cast<double*>(roff + TILE_R);
+        ++nr;
+        // a real alpha that is a power of two is folded into the row factor (exact, so the result equals the validation
+        // engine's alpha * value)
+        const double al = q.alpha_pow2 ? q.alpha.x : 1.0;
+        const int32_t* eB = q.eB + w.rbB * q.eB_ld + row0;
+        int e[TILE_R / 32];
+#pragma unroll
+        for (int j = 0; j < TILE_R / 32; ++j) e[j] = lane + 32 * j < rlim ? eB[lane + 32 * j] : 0;
+#pragma unroll
+        for (int j = 0; j < TILE_R / 32; ++j) {
+          const int i = lane + 32 * j;
+          roff[i] = i < rlim ? q.C.col(row0 + i) : 0;
+          rsc[i] = pow2(e[j]) * al;
         }
       }
-      if (et == 0) {
-        const bool ok = mbar_wait(&accf_bar[buf], (uint32_t)(use & 1), abort_flag);
-        if (!ok) {
+      if (lane < q.BN / 2) {
+        coff[lane] = o0;
+        csc[lane] = pow2(e0 - unit_exp(S));
+      }
+      for (int i = lane + 32; i < q.BN / 2; i += 32) {
+        const bool in = i < clim;
+        coff[i] = in ? q.C.row(m0 + i) : 0;
+        csc[i] = pow2((in ? eA[i] : 0) - unit_exp(S));
+      }
+      if (lane == 0) {
+        TileHead& h = *reinterpret_cast<TileHead*>(tb);
+        h.C = q.C.ptr + q.C.bat(w.b0, w.b1, w.b2);
+        h.rlim = (int)(rlim < TILE_R ? rlim : TILE_R);
+        h.clim = (int)(clim < q.BN / 2 ? clim : q.BN / 2);
+        h.ngroups = (2 * h.clim + EPI_CG - 1) / EPI_CG;
+        h.bn = q.BN;
+        h.rowset = (int)((nr - 1) & 1);
+        h.scaled = !q.alpha_pow2;
+        h.has_beta = q.beta.x != 0.0 || q.beta.y != 0.0;
+        h.alpha = q.alpha;
+        h.beta = q.beta;
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive_local(&tabf_bar[set]);
+    }
+  } else {
+    // epilogue warps: TMEM sub-partition = warp % 4, one row of the tile per lane; the EPI_WARPS / 4 warps of a
+    // sub-partition take the groups of EPI_CG columns in turn.
+    const int sp = warp % 4;
+    const int row = sp * 32 + lane;
+    uint32_t tcount = 0, acc_ph = 0, turn = (uint32_t)(warp - EPI_FIRST) / 4;
+    int buf = 0;
+    for (uint32_t t = t_first; t < t_end; t += t_step, ++tcount) {
+      const int set = (int)(tcount & 1);
+      bool ok = true;
+      if (lane == 0)
+        ok = mbar_wait(&tabf_bar[set], (tcount >> 1) & 1, abort_flag) && mbar_wait(&accf_bar[buf], acc_ph, abort_flag);
+      if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) {
+        if (lane == 0) {
           atomicExch(p.err, SERR_TIMEOUT_EPILOGUE);
           *abort_flag = 1;
         }
-        epi_ok[tcount & 1] = ok ? 1 : 0;
+        break;
       }
-      // every epilogue thread reaches every named barrier, on the error path too
-      epi_bar();
-      if (!epi_ok[tcount & 1]) break;
       tc_fence_after();
-      // a real alpha that is a power of two is folded into the row factor (exact, so the result
-      // equals the validation engine's alpha * value); the store is then a plain copy
-      const bool alpha_in_tile = q.alpha_pow2 != 0;
-      const double rs = alpha_in_tile ? pow2(sh_eA[mloc]) * q.alpha.x : pow2(sh_eA[mloc]);
-      // a warp whose 32 rows are all padding skips the accumulator reads
-      const bool live = tc.mrow0 + sp * 32 < 2 * q.M;
+      const uint8_t* tb = tables + set * tsb;
+      const TileHead& h = *reinterpret_cast<const TileHead*>(tb);
+      const int64_t* roff = reinterpret_cast<const int64_t*>(row_tables + h.rowset * ROW_TABLE_BYTES);
+      const double* rsc = reinterpret_cast<const double*>(roff + TILE_R);
+      const int bn = h.bn, clim = h.clim;
+      const int64_t* coff = reinterpret_cast<const int64_t*>(tb + sizeof(TileHead));
+      const double* csc = reinterpret_cast<const double*>(coff + bn / 2);
+      // a warp whose 32 rows all lie outside the result has no groups
+      const int ng = sp * 32 < h.rlim ? h.ngroups : 0;
+      const bool rok = row < h.rlim;
+      const double rs = rsc[row];
+      cplx* Crow = h.C + roff[row];
+      const bool plain = !h.scaled && !h.has_beta;
       const uint32_t acc = tmem_base + (uint32_t)buf * acc_cols + ((uint32_t)(sp * 32) << 16);
-      const int64_t mlim = q.M - tc.mrow0 / 2, nlim = q.N - tc.ncol0;
-      const bool mok = mloc < mlim;
-      cplx* Crow = q.C.ptr + q.C.bat(tc.b0, tc.b1, tc.b2) + sh_rowC[mloc];
-      const bool has_beta = q.beta.x != 0.0 || q.beta.y != 0.0;
-      for (int c0 = 0; c0 < q.BN; c0 += EPI_CH) {
-        const int cw = min(EPI_CH, q.BN - c0);
-        const int cc = grp * EPI_CG;
-        const bool last = c0 + EPI_CH >= q.BN;
-        double v[EPI_CG];
-        const bool work = live && cc < cw;
-        if (work) {
-          // all S diagonals of the warp's 8 columns in one TMEM round trip
-          int32_t dq[S][1][EPI_CG];
+      // the first group rotates, so that a group count that is no multiple of four loads the warps evenly
+      const int gfirst = (int)(turn & 3u);
+      turn += (uint32_t)(bn / EPI_CG);
+      for (int g = gfirst; g < ng; g += EPI_WARPS / 4) {
+        // all S diagonals of 8 columns in one TMEM round trip
+        int32_t dq[S][EPI_CG];
 #pragma unroll
-          for (int d = 0; d < S; ++d) tmem_ld8(acc + (uint32_t)(d * q.BN + c0 + cc), dq[d][0]);
-          tmem_wait_ld();
-          combine_cols<S, EPI_CG>(dq, q.pair != 0, v);
+        for (int d = 0; d < S; ++d) tmem_ld8(acc + (uint32_t)(d * bn + g * EPI_CG), dq[d]);
+        tmem_wait_ld();
+        cplx v[EPI_CG / 2];
+#pragma unroll
+        for (int j = 0; j < EPI_CG / 2; ++j) {
+          int32_t qr[S], qi[S];
+#pragma unroll
+          for (int d = 0; d < S; ++d) {
+            qr[d] = dq[d][2 * j];
+            qi[d] = dq[d][2 * j + 1];
+          }
+          const double sc = rs * csc[g * (EPI_CG / 2) + j];
+          v[j] = cmk(combine_diagonals<S>(qr) * sc, combine_diagonals<S>(qi) * sc);
         }
-        if (last) {
-          // this warp's reads of the accumulator set are complete: release it to the MMA warp
+        if (g + EPI_WARPS / 4 >= ng) {
+          // this warp's reads of the accumulators are complete: release them to the MMA warp
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive_local(&acce_bar[buf]);
         }
-        if (work) {
+        const int c0 = g * (EPI_CG / 2);
+        if (rok) {
+          if (plain) {
 #pragma unroll
-          for (int j = 0; j < EPI_CG; ++j) v[j] *= rs * sh_csc[c0 + cc + j];
-          // the even lane keeps columns [0, H) of the group, the odd lane [H, 2H)
-          double other[H];
+            for (int j = 0; j < EPI_CG / 2; ++j)
+              if (c0 + j < clim) Crow[coff[c0 + j]] = v[j];
+          } else {
 #pragma unroll
-          for (int i = 0; i < H; ++i) other[i] = __shfl_xor_sync(0xffffffffu, r ? v[i] : v[H + i], 1);
-          if (mok) {
-#pragma unroll
-            for (int i = 0; i < H; ++i) {
-              const int col = c0 + cc + (r ? H + i : i);
-              if (col < nlim) {
-                cplx* d = Crow + sh_colC[col];
-                cplx val = r ? cmk(other[i], v[H + i]) : cmk(v[i], other[i]);
-                if (!alpha_in_tile) val = cmul(q.alpha, val);
-                if (has_beta) val = cadd(val, cmul(q.beta, *d));
+            for (int j = 0; j < EPI_CG / 2; ++j)
+              if (c0 + j < clim) {
+                cplx* d = Crow + coff[c0 + j];
+                cplx val = h.scaled ? cmul(h.alpha, v[j]) : v[j];
+                if (h.has_beta) val = cadd(val, cmul(h.beta, *d));
                 *d = val;
               }
-            }
-          }
-          if constexpr (SINK) {
-            if (q.sink.expo) {
-              // exponent of the largest stored |Re|, |Im| of the warp's 8 columns (one aligned group,
-              // one entry), with the convention of slice_expo_kernel; the host allows sinks only
-              // where the stored value is v itself (alpha a power of two folded into rs, beta = 0)
-              double smax = 0.0;
-              if (mok) {
-#pragma unroll
-                for (int j = 0; j < EPI_CG; ++j)
-                  if (c0 + cc + j < nlim) smax = fmax(smax, fabs(v[j]));
-              }
-              int ev = INT_MIN;
-              if (smax > 0.0) {
-                const int biased = (int)((__double_as_longlong(smax) >> 52) & 0x7FF);
-                int ex = biased - 1022;  // frexp's exponent for a normal number
-                if (biased == 0) frexp(smax, &ex);
-                ev = ex + 1;
-              }
-              ev = __reduce_max_sync(0xffffffffu, ev);
-              if (lane == 0 && ev != INT_MIN) atomicMax(q.sink.expo + sh_key[(c0 + cc) / EPI_CG], ev);
-            }
           }
         }
+      }
+      if (gfirst >= ng) {  // no group of this tile was this warp's
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_local(&acce_bar[buf]);
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive_local(&tabe_bar[set]);
+      if (++buf == nbuf) {
+        buf = 0;
+        acc_ph ^= 1;
       }
     }
   }
@@ -940,11 +1050,15 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
   __syncthreads();
   // after an abort, let in-flight TMA loads land before the shared memory is released
   if (warp == 0 && lane == 0 && *abort_flag) {
-    for (int64_t k = (issued > L.stages ? issued - L.stages : 0); k < issued; ++k) {
-      long long t0 = clock64();
-      while (!mbar_try_wait(&full_bar[k % L.stages], (uint32_t)((k / L.stages) & 1))) {
+    for (uint32_t k = (issued > (uint32_t)nstage ? issued - nstage : 0); k < issued; ++k) {
+      const long long t0 = clock64();
+      while (!mbar_try_wait(&full_bar[k % nstage], (k / nstage) & 1))
         if (clock64() - t0 > WAIT_LIMIT) break;
-      }
+    }
+    for (uint32_t k = (nrows > 2 ? nrows - 2 : 0); k < nrows; ++k) {
+      const long long t0 = clock64();
+      while (!mbar_try_wait(&rowf_bar[k & 1], (k >> 1) & 1))
+        if (clock64() - t0 > WAIT_LIMIT) break;
     }
   }
   __syncthreads();
@@ -957,6 +1071,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
 // ----------------------------------------------------------------------------
 // CUDA-core validation core: the same diagonal INT32 sums from the same planes.
 // ----------------------------------------------------------------------------
+template <int S>
 __global__ void split_gemm_ref_kernel(const int8_t* Ap, const int8_t* Bp, int64_t kpad, GemmParams p) {
   const int64_t bz = blockIdx.z;
   const int64_t b2 = bz % p.nb2, b1 = (bz / p.nb2) % p.nb1, b0 = bz / (p.nb2 * p.nb1);
@@ -965,15 +1080,14 @@ __global__ void split_gemm_ref_kernel(const int8_t* Ap, const int8_t* Bp, int64_
   const int64_t m = (int64_t)blockIdx.y * 16 + threadIdx.y;
   const int64_t n = (int64_t)blockIdx.x * 16 + threadIdx.x;
   if (m >= p.M || n >= p.N) return;
-  const int S = p.S;
-  int32_t qr[8], qi[8];
+  int32_t qr[S], qi[S];
+#pragma unroll
   for (int d = 0; d < S; ++d) {
     int32_t accr = 0, acci = 0;
     for (int s = 0; s <= d; ++s) {
-      const int t = d - s;
-      const int8_t* a0 = Ap + ((rbA * S + s) * p.rowsA_pad + 2 * m) * kpad;
+      const int8_t* a0 = Ap + ((rbA * S + s) * p.rowsA + 2 * m) * kpad;
       const int8_t* a1 = a0 + kpad;
-      const int8_t* bb = Bp + ((rbB * S + t) * p.rowsB_pad + n) * kpad;
+      const int8_t* bb = Bp + ((rbB * S + d - s) * p.rowsB + n) * kpad;
       for (int64_t k = 0; k < kpad; ++k) {
         accr += (int32_t)a0[k] * (int32_t)bb[k];
         acci += (int32_t)a1[k] * (int32_t)bb[k];
@@ -982,8 +1096,11 @@ __global__ void split_gemm_ref_kernel(const int8_t* Ap, const int8_t* Bp, int64_
     qr[d] = accr;
     qi[d] = acci;
   }
-  const double re = combine_diagonals(qr, S), im = combine_diagonals(qi, S);
-  store_result(p, b0, b1, b2, m, n, re, im, p.eA[rbA * p.eA_ld + m], p.eB[rbB * p.eB_ld + n]);
+  const double sc = pow2(p.eB[rbB * p.eB_ld + n]) * pow2(p.eA[rbA * p.eA_ld + m] - unit_exp(S));
+  cplx* dst = p.C.ptr + p.C.bat(b0, b1, b2) + p.C.row(m) + p.C.col(n);
+  cplx v = cmul(p.alpha, cmk(combine_diagonals<S>(qr) * sc, combine_diagonals<S>(qi) * sc));
+  if (p.beta.x != 0.0 || p.beta.y != 0.0) v = cadd(v, cmul(p.beta, *dst));
+  *dst = v;
 }
 
 // ----------------------------------------------------------------------------
@@ -1003,15 +1120,16 @@ PFN_cuTensorMapEncodeTiled_v12000 get_encode() {
   return fn;
 }
 
-CUtensorMap make_map(const int8_t* base, int64_t kpad, int64_t rows_total, int box_rows) {
+// planes [nplanes][rows][kpad] of an operand; a load takes box_rows rows of one K block from S planes
+CUtensorMap make_map(const int8_t* base, int64_t kpad, int64_t rows, int64_t nplanes, int box_rows, int S) {
   CUtensorMap m;
   std::memset(&m, 0, sizeof(m));
-  cuuint64_t dims[2] = {(cuuint64_t)kpad, (cuuint64_t)rows_total};
-  cuuint64_t strides[1] = {(cuuint64_t)kpad};
-  cuuint32_t box[2] = {(cuuint32_t)KBLK, (cuuint32_t)box_rows};
-  cuuint32_t estr[2] = {1, 1};
+  cuuint64_t dims[3] = {(cuuint64_t)kpad, (cuuint64_t)rows, (cuuint64_t)nplanes};
+  cuuint64_t strides[2] = {(cuuint64_t)kpad, (cuuint64_t)(kpad * rows)};
+  cuuint32_t box[3] = {(cuuint32_t)KBLK, (cuuint32_t)box_rows, (cuuint32_t)S};
+  cuuint32_t estr[3] = {1, 1, 1};
   require((reinterpret_cast<uintptr_t>(base) & 15) == 0 && kpad % 16 == 0, GB200_ERR_INVALID, "TMA alignment");
-  CUresult r = get_encode()(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(base), dims, strides, box, estr,
+  CUresult r = get_encode()(&m, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t*>(base), dims, strides, box, estr,
                             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   require(r == CUDA_SUCCESS, GB200_ERR_CUDA, "cuTensorMapEncodeTiled failed");
@@ -1101,12 +1219,12 @@ void launch_resident(const SliceJob& j, dim3 g, size_t sm, int kt, cudaStream_t 
 void set_smem_attrs(SplitEngine& se) {
   if (se.attr_set) return;
   const void* fns[] = {
-#define GB_TC_ALL(G, K)                                                                    \
-  (const void*)split_gemm_tc_kernel<2, G, K>, (const void*)split_gemm_tc_kernel<3, G, K>, \
-      (const void*)split_gemm_tc_kernel<4, G, K>, (const void*)split_gemm_tc_kernel<5, G, K>, \
-      (const void*)split_gemm_tc_kernel<6, G, K>, (const void*)split_gemm_tc_kernel<7, G, K>, \
-      (const void*)split_gemm_tc_kernel<8, G, K>
-      GB_TC_ALL(false, false), GB_TC_ALL(false, true), GB_TC_ALL(true, false), GB_TC_ALL(true, true),
+#define GB_TC_ALL(G)                                                                                     \
+  (const void*)split_gemm_tc_kernel<2, G>, (const void*)split_gemm_tc_kernel<3, G>,                      \
+      (const void*)split_gemm_tc_kernel<4, G>, (const void*)split_gemm_tc_kernel<5, G>,                  \
+      (const void*)split_gemm_tc_kernel<6, G>, (const void*)split_gemm_tc_kernel<7, G>,                  \
+      (const void*)split_gemm_tc_kernel<8, G>
+      GB_TC_ALL(false), GB_TC_ALL(true),
 #undef GB_TC_ALL
 #define GB_RES_ALL(RB)                                                                        \
   (const void*)slice_resident_kernel<RB, 2>, (const void*)slice_resident_kernel<RB, 3>,       \
@@ -1162,43 +1280,40 @@ void run_slicer(SliceJob& j, int64_t nrb, cudaStream_t st) {
   GB_CHECK_LAUNCH();
 }
 
-// The digit pass alone, with the exponents already in j.expo (empty rows marked EXP_EMPTY).
-void run_slicer_known_expo(SliceJob& j, int64_t nrb, cudaStream_t st) {
-  require(nrb < 65536, GB200_ERR_INVALID, "split: too many operand batches");
-  j.single = 0;
-  dim3 g((unsigned)((j.rpad + TR - 1) / TR), (unsigned)((j.kpad / 2 + TK - 1) / TK), (unsigned)nrb);
-  require(g.y < 65536, GB200_ERR_INVALID, "split: contraction too long for the slicer grid");
-  launch_write(j, g, st);
-  GB_CHECK_LAUNCH();
-  fix_empty_expo_kernel<<<blocks_for(nrb * j.e_ld), 256, 0, st>>>(j.expo, nrb * j.e_ld);
-  GB_CHECK_LAUNCH();
-}
-
 }  // namespace
 
 namespace {
 
-// largest K chunk for which no INT32 diagonal can overflow: S * 2K * 127^2 < 2^31
+// largest K chunk for which no INT32 diagonal can overflow: S * 2K * 128^2 < 2^31 (base 128: 64^2 at most)
 int64_t kmax_for(int S) {
-  int64_t kmax = (int64_t)(2147483647.0 / (2.0 * 127.0 * 127.0 * S));
+  int64_t kmax = (int64_t)(2147483647.0 / (2.0 * 128.0 * 128.0 * S));
   return kmax / 32 * 32;
 }
 
-// Tile width of a problem: one TMEM accumulator set of up to 512 columns and the widest tile it
-// allows, or the context's chosen width.  Measured on B200 for every launch shape of the GW
-// chain, one set of the widest tile is faster than two sets of half the width (the epilogue of
-// one tile overlapping the next tile's MMAs), with one MMA per slice product or with one MMA of
-// width (S - s) BN per A slice plane: narrower tiles double the per-tile epilogue work (tables,
-// barrier, TMEM round trips) that dominates the short contractions.
-int tile_width(const Context& c, int S, int64_t N) {
-  int bn = max_bn(S, 512);
-  if (c.tile_bn > 0) bn = std::min(bn, std::max(16, c.tile_bn / 16 * 16));
-  return std::min<int>(bn, (int)rup(N, 16));
+// Tile width of a problem, in real columns of the embedded operand (2 M of them): one TMEM accumulator set of up to 512
+// columns (two of half that in overlap mode), or the context's chosen width, and below that the multiple of 16 with
+// which the tiles cost least: a K step moves the planes of 128 rows and BN columns from L2 (33 bytes a cycle and SM
+// measured), which takes longer than its MMAs; in overlap mode a tile costs its epilogue and about 16 columns' worth
+// of waits.
+int tile_width(const Context& c, int S, int64_t M, bool overlap) {
+  int top = max_bn(S, overlap ? 256 : 512);
+  if (c.tile_bn > 0) top = std::min(top, std::max(16, c.tile_bn / 16 * 16));
+  top = std::min<int>(top, (int)std::min<int64_t>(rup(2 * M, 16), 256));
+  int best = top;
+  double cost = 1e300;
+  for (int bn = top; bn >= 16 && 2 * bn >= top; bn -= 16) {
+    const double x = std::ceil(2.0 * (double)M / bn) * (bn + (overlap ? 16.0 : (double)TILE_R));
+    if (x < cost) {
+      cost = x;
+      best = bn;
+    }
+  }
+  return best;
 }
 
 struct Prepared {
   GemmParams p{};
-  CUtensorMap mA{}, mB{};
+  CUtensorMap mR{}, mC{};
   int64_t kpad = 0, ntiles = 0;
   double flops = 0.0;
 };
@@ -1212,139 +1327,101 @@ Prepared prepare_chunk(SplitEngine& se, const ZGemm& g0, int S, int BN, int64_t 
   deps_of(g0.A, depA);
   deps_of(g0.B, depB);
   const int64_t nrbA = nrb_of(depA, g0), nrbB = nrb_of(depB, g0);
-  const int64_t rowsA_pad = rup(2 * g0.M, TILE_M);
-  const int64_t rowsB_pad = rup(g0.N, BN);
+  const int64_t rowsA = 2 * g0.M, rowsB = g0.N;
   if (!se.err.p) {
     se.err.alloc(1);
     GB_CUDA(cudaMemsetAsync(se.err.p, 0, sizeof(int), st));
   }
-  const int64_t kpad = rup(2 * Kc, KBLK);
-  se.planesA.alloc((size_t)(nrbA * S * rowsA_pad * kpad));
-  se.planesB.alloc((size_t)(nrbB * S * rowsB_pad * kpad));
-  se.expA.alloc((size_t)(nrbA * rowsA_pad / 2));
-  se.expB.alloc((size_t)(nrbB * rowsB_pad));
-  {
+  // whole 32-byte K steps of the MMA; a last half block is filled with zeros by the TMA load
+  const int64_t kpad = std::max<int64_t>(KBLK, rup(2 * Kc, 32));
+  se.planesA.alloc((size_t)(nrbA * S * rowsA * kpad));
+  se.planesB.alloc((size_t)(nrbB * S * rowsB * kpad));
+  se.expA.alloc((size_t)(nrbA * g0.M));
+  se.expB.alloc((size_t)(nrbB * g0.N));
+  auto slice = [&](const ZOperand& o, const IdxMap& rmap, const IdxMap& kmap, const int* dep, int64_t R, int64_t nrb,
+                   int embed, int8_t* out, int32_t* expo) {
     SliceJob j{};
-    j.ptr = g0.A.ptr; j.rmap = g0.A.row; j.kmap = g0.A.col; j.bat = g0.A.bat; j.conj = g0.A.conj;
-    j.R = g0.M; j.K = Kc; j.k0 = k0; j.n0 = g0.nb0; j.n1 = g0.nb1; j.n2 = g0.nb2;
-    std::copy(depA, depA + 3, j.dep);
-    j.embed = 1; j.S = S; j.rows_pad = rowsA_pad; j.rpad = rowsA_pad / 2; j.kpad = kpad; j.e_ld = rowsA_pad / 2;
-    j.out = se.planesA.p; j.expo = se.expA.p;
-    j.r_fast = std::abs(g0.A.row.s_in) < std::abs(g0.A.col.s_in);
-    run_slicer(j, nrbA, st);
-  }
-  {
-    SliceJob j{};
-    // right operand sliced per column: the job's rows are the N columns, K runs along B's rows
-    j.ptr = g0.B.ptr; j.rmap = g0.B.col; j.kmap = g0.B.row; j.bat = g0.B.bat; j.conj = g0.B.conj;
-    j.R = g0.N; j.K = Kc; j.k0 = k0; j.n0 = g0.nb0; j.n1 = g0.nb1; j.n2 = g0.nb2;
-    std::copy(depB, depB + 3, j.dep);
-    j.embed = 0; j.S = S; j.rows_pad = rowsB_pad; j.rpad = rowsB_pad; j.kpad = kpad; j.e_ld = rowsB_pad;
-    j.out = se.planesB.p; j.expo = se.expB.p;
-    j.r_fast = std::abs(g0.B.col.s_in) < std::abs(g0.B.row.s_in);
-    if (g0.B_expo) {
-      // the producer of B recorded its column exponents (over the whole K range, so every chunk
-      // can use them): only the digit pass runs
-      require(g0.B_expo_ld >= g0.N, GB200_ERR_INVALID, "split: exponent array of B too short");
-      j.expo = g0.B_expo;
-      j.e_ld = g0.B_expo_ld;
-      run_slicer_known_expo(j, nrbB, st);
-    } else {
-      run_slicer(j, nrbB, st);
-    }
-  }
-  if (g0.sink.expo) {
-    int aexp = 0;
-    require(se.core == 0, GB200_ERR_INVALID, "split: exponent sinks need the tensor-core engine");
-    require(k0 == 0 && Kc == g0.K, GB200_ERR_INVALID, "split: an exponent sink needs a single K chunk");
-    require(g0.beta.x == 0.0 && g0.beta.y == 0.0 && g0.alpha.y == 0.0 && g0.alpha.x != 0.0 &&
-                std::fabs(std::frexp(g0.alpha.x, &aexp)) == 0.5,
-            GB200_ERR_INVALID, "split: an exponent sink needs beta = 0 and a real power-of-two alpha");
-    require((g0.sink.s1 == 0 || g0.sink.d1 % 8 == 0) && (g0.sink.s2 == 0 || g0.sink.d2 % 8 == 0), GB200_ERR_INVALID,
-            "split: sink entries must be constant over aligned groups of 8 columns");
-    require(g0.sink.count < (1LL << 31), GB200_ERR_INVALID, "split: exponent sink too large");
-    fill_int_kernel<<<blocks_for(g0.sink.count), 256, 0, st>>>(g0.sink.expo, g0.sink.count, EXP_EMPTY);
-    GB_CHECK_LAUNCH();
-  }
+    j.ptr = o.ptr; j.rmap = rmap; j.kmap = kmap; j.bat = o.bat; j.conj = o.conj;
+    j.R = R; j.K = Kc; j.k0 = k0; j.n0 = g0.nb0; j.n1 = g0.nb1; j.n2 = g0.nb2;
+    std::copy(dep, dep + 3, j.dep);
+    j.embed = embed; j.S = S; j.rows_pad = embed ? 2 * R : R; j.rpad = R; j.kpad = kpad; j.e_ld = R;
+    j.out = out; j.expo = expo;
+    j.r_fast = std::abs(rmap.s_in) < std::abs(kmap.s_in);
+    run_slicer(j, nrb, st);
+  };
+  slice(g0.A, g0.A.row, g0.A.col, depA, g0.M, nrbA, 1, se.planesA.p, se.expA.p);
+  slice(g0.B, g0.B.col, g0.B.row, depB, g0.N, nrbB, 0, se.planesB.p, se.expB.p);
   GemmParams& p = pr.p;
-  p.S = S; p.BN = BN; p.nkb = (int)(kpad / KBLK);
+  p.S = S; p.BN = BN; p.nkb = (int)((kpad + KBLK - 1) / KBLK); p.nkk = (int)(kpad / 32);
   p.M = g0.M; p.N = g0.N; p.nb0 = g0.nb0; p.nb1 = g0.nb1; p.nb2 = g0.nb2;
   std::copy(depA, depA + 3, p.depA);
   std::copy(depB, depB + 3, p.depB);
-  p.rowsA_pad = rowsA_pad; p.rowsB_pad = rowsB_pad;
-  p.eA = se.expA.p; p.eB = se.expB.p; p.eA_ld = rowsA_pad / 2; p.eB_ld = rowsB_pad;
-  if (g0.B_expo) {
-    p.eB = g0.B_expo;
-    p.eB_ld = g0.B_expo_ld;
-  }
-  p.sink = g0.sink;
+  p.rowsA = rowsA; p.rowsB = rowsB;
+  p.eA = se.expA.p; p.eB = se.expB.p; p.eA_ld = g0.M; p.eB_ld = g0.N;
   p.C = g0.C; p.alpha = g0.alpha; p.beta = (k0 == 0) ? g0.beta : cmk(1.0, 0.0);
   p.err = se.err.p;
   {
     int aexp = 0;
     p.alpha_pow2 = (g0.alpha.y == 0.0 && g0.alpha.x != 0.0 && std::fabs(std::frexp(g0.alpha.x, &aexp)) == 0.5) ? 1 : 0;
   }
-  {
-    // |q_d| <= (d + 1) * 2Kc * 64^2 (d + 1 digit pairs per diagonal, balanced digits |q| <= 64):
-    // pair (d, d + 1) is exact in int32 when 128 max|q_d| + max|q_(d+1)| < 2^31
-    bool ok = S <= 5;
-    for (int d = 0; ok && d + 1 < S && d <= 2; d += 2)
-      ok = 2.0 * (double)Kc * 4096.0 * (128.0 * (d + 1) + (d + 2)) < 2147483648.0;
-    p.pair = ok ? 1 : 0;
-  }
-  p.rows_fast = std::abs(g0.C.row.s_in) < std::abs(g0.C.col.s_in) ? 1 : 0;
   const int64_t nbatch = g0.nb0 * g0.nb1 * g0.nb2;
   require(nbatch < 65536, GB200_ERR_INVALID, "split: too many batches for one launch");
-  p.tiles_m = (int)(rowsA_pad / TILE_M);
-  p.tiles_n = (int)(rowsB_pad / BN);
+  p.tiles_r = (int)((g0.N + TILE_R - 1) / TILE_R);
+  p.tiles_c = (int)((rowsA + BN - 1) / BN);
   pr.kpad = kpad;
-  pr.ntiles = (int64_t)p.tiles_m * p.tiles_n * nbatch;
+  pr.ntiles = (int64_t)p.tiles_r * p.tiles_c * nbatch;
+  require(pr.ntiles < (1LL << 31), GB200_ERR_INVALID, "split: too many tiles for one launch");
+  p.ntile = (int)pr.ntiles;
   pr.flops = 8.0 * (double)g0.M * (double)g0.N * (double)Kc * (double)nbatch;
   if (se.core == 0) {
-    const int64_t rowsA_total = nrbA * S * rowsA_pad;
-    const int64_t rowsB_total = nrbB * S * rowsB_pad;
-    require(rowsA_total < (1LL << 31) && rowsB_total < (1LL << 31), GB200_ERR_INVALID, "split: operand too large for TMA");
-    pr.mA = make_map(se.planesA.p, kpad, rowsA_total, TILE_M);
-    pr.mB = make_map(se.planesB.p, kpad, rowsB_total, BN);
+    const int64_t totalA = nrbA * S * rowsA, totalB = nrbB * S * rowsB;
+    require(totalA < (1LL << 31) && totalB < (1LL << 31), GB200_ERR_INVALID, "split: operand too large for TMA");
+    pr.mR = make_map(se.planesB.p, kpad, rowsB, nrbB * S, TILE_R, S);
+    pr.mC = make_map(se.planesA.p, kpad, rowsA, nrbA * S, BN, S);
   }
   return pr;
 }
 
-template <bool G, bool K>
-void launch_tc_s(int S, unsigned grid, size_t smem, cudaStream_t st, const CUtensorMap& mA, const CUtensorMap& mB,
-                 const GemmParams& p) {
+template <bool G>
+void launch_tc(int S, unsigned grid, size_t smem, cudaStream_t st, const CUtensorMap& mR, const CUtensorMap& mC,
+               const GemmParams& p) {
   switch (S) {
-    case 2: split_gemm_tc_kernel<2, G, K><<<grid, NWARPS * 32, smem, st>>>(mA, mB, p); break;
-    case 3: split_gemm_tc_kernel<3, G, K><<<grid, NWARPS * 32, smem, st>>>(mA, mB, p); break;
-    case 4: split_gemm_tc_kernel<4, G, K><<<grid, NWARPS * 32, smem, st>>>(mA, mB, p); break;
-    case 5: split_gemm_tc_kernel<5, G, K><<<grid, NWARPS * 32, smem, st>>>(mA, mB, p); break;
-    case 6: split_gemm_tc_kernel<6, G, K><<<grid, NWARPS * 32, smem, st>>>(mA, mB, p); break;
-    case 7: split_gemm_tc_kernel<7, G, K><<<grid, NWARPS * 32, smem, st>>>(mA, mB, p); break;
-    default: split_gemm_tc_kernel<8, G, K><<<grid, NWARPS * 32, smem, st>>>(mA, mB, p); break;
+    case 2: split_gemm_tc_kernel<2, G><<<grid, NWARPS * 32, smem, st>>>(mR, mC, p); break;
+    case 3: split_gemm_tc_kernel<3, G><<<grid, NWARPS * 32, smem, st>>>(mR, mC, p); break;
+    case 4: split_gemm_tc_kernel<4, G><<<grid, NWARPS * 32, smem, st>>>(mR, mC, p); break;
+    case 5: split_gemm_tc_kernel<5, G><<<grid, NWARPS * 32, smem, st>>>(mR, mC, p); break;
+    case 6: split_gemm_tc_kernel<6, G><<<grid, NWARPS * 32, smem, st>>>(mR, mC, p); break;
+    case 7: split_gemm_tc_kernel<7, G><<<grid, NWARPS * 32, smem, st>>>(mR, mC, p); break;
+    default: split_gemm_tc_kernel<8, G><<<grid, NWARPS * 32, smem, st>>>(mR, mC, p); break;
   }
   GB_CHECK_LAUNCH();
 }
 
-// `sink`: some problem of the launch records exponents (otherwise the kernel without that code)
-template <bool G>
-void launch_tc(int S, bool sink, unsigned grid, size_t smem, cudaStream_t st, const CUtensorMap& mA,
-               const CUtensorMap& mB, const GemmParams& p) {
-  if (sink) launch_tc_s<G, true>(S, grid, smem, st, mA, mB, p);
-  else launch_tc_s<G, false>(S, grid, smem, st, mA, mB, p);
+void launch_ref(int S, dim3 grid, cudaStream_t st, const int8_t* A, const int8_t* B, int64_t kpad, const GemmParams& p) {
+  const dim3 block(16, 16);
+  switch (S) {
+    case 2: split_gemm_ref_kernel<2><<<grid, block, 0, st>>>(A, B, kpad, p); break;
+    case 3: split_gemm_ref_kernel<3><<<grid, block, 0, st>>>(A, B, kpad, p); break;
+    case 4: split_gemm_ref_kernel<4><<<grid, block, 0, st>>>(A, B, kpad, p); break;
+    case 5: split_gemm_ref_kernel<5><<<grid, block, 0, st>>>(A, B, kpad, p); break;
+    case 6: split_gemm_ref_kernel<6><<<grid, block, 0, st>>>(A, B, kpad, p); break;
+    case 7: split_gemm_ref_kernel<7><<<grid, block, 0, st>>>(A, B, kpad, p); break;
+    default: split_gemm_ref_kernel<8><<<grid, block, 0, st>>>(A, B, kpad, p); break;
+  }
+  GB_CHECK_LAUNCH();
 }
 
 // Launch-wide layout for tiles up to BN columns: TMA ring depth (what fits, at most 6 K blocks)
 // and the dynamic shared memory.
 void ring_layout(int S, int BN, GemmParams& p, size_t& smem) {
-  const SmemLayout L1 = smem_layout(S, BN, 1);
-  int stages = (SMEM_BUDGET - L1.ctile_bytes - 4096) / L1.stage_bytes;
-  stages = std::max(1, std::min(stages, 6));
-  p.stages = stages;
-  p.nbuf = 1;
-  const SmemLayout Ls = smem_layout(S, BN, stages);
-  smem = (size_t)Ls.ring_bytes + Ls.ctile_bytes + 1024 /*alignment*/ + misc_bytes(stages, BN);
-  require(smem <= 227 * 1024, GB200_ERR_INVALID, "split: shared memory budget exceeded");
+  const SmemLayout L1 = smem_layout(S, BN, 1, p.overlap);
+  const int room = SMEM_MAX - 1024 /*alignment*/ - misc_bytes(6, BN) - L1.rows_bytes;
+  p.stages = std::max(1, std::min(room / L1.stage_bytes, 6));
+  smem = (size_t)smem_layout(S, BN, p.stages, p.overlap).ring_bytes + 1024 + misc_bytes(p.stages, BN);
+  require(smem <= SMEM_MAX, GB200_ERR_INVALID, "split: shared memory budget exceeded");
 }
+
+bool overlap_mode(int S, int64_t K) { return S <= OVERLAP_MAX_S && 2 * K <= RES_KB * KBLK; }
 
 KernelRecord* begin_record(Context& c, double flops, cudaStream_t st) {
   if (!c.stats_on) return nullptr;
@@ -1375,7 +1452,8 @@ void split_gemm(Context& c, SplitEngine& se, const ZGemm& g0, cudaStream_t st, i
   const int S = slices > 0 ? slices : c.slices;
   require(S >= 2 && S <= 8, GB200_ERR_INVALID, "split: slices out of range");
   require(g0.K > 0, GB200_ERR_INVALID, "split: empty contraction");
-  const int BN = tile_width(c, S, g0.N);
+  const bool overlap = overlap_mode(S, g0.K);
+  const int BN = tile_width(c, S, g0.M, overlap);
   const int64_t kmax = kmax_for(S);
   for (int64_t k0 = 0; k0 < g0.K; k0 += kmax) {
     const int64_t Kc = std::min(kmax, g0.K - k0);
@@ -1383,19 +1461,17 @@ void split_gemm(Context& c, SplitEngine& se, const ZGemm& g0, cudaStream_t st, i
     const int64_t nbatch = g0.nb0 * g0.nb1 * g0.nb2;
     if (se.core == 1) {
       dim3 grid((unsigned)((g0.N + 15) / 16), (unsigned)((g0.M + 15) / 16), (unsigned)nbatch);
-      split_gemm_ref_kernel<<<grid, dim3(16, 16), 0, st>>>(se.planesA.p, se.planesB.p, pr.kpad, pr.p);
-      GB_CHECK_LAUNCH();
+      launch_ref(S, grid, st, se.planesA.p, se.planesB.p, pr.kpad, pr.p);
       continue;
     }
     size_t smem = 0;
+    pr.p.overlap = overlap ? 1 : 0;
     ring_layout(S, BN, pr.p, smem);
     KernelRecord* rec = begin_record(c, pr.flops, st);
-    launch_tc<false>(S, pr.p.sink.expo != nullptr, persistent_grid(c, pr.ntiles), smem, st, pr.mA, pr.mB, pr.p);
+    launch_tc<false>(S, persistent_grid(c, pr.ntiles), smem, st, pr.mR, pr.mC, pr.p);
     if (rec) GB_CUDA(cudaEventRecord(rec->stop, st));
   }
 }
-
-int64_t split_max_chunk(int slices) { return kmax_for(slices); }
 
 void split_gemm_group(const std::vector<Context*>& cs, const std::vector<ZGemm>& gs, cudaStream_t st, int slices) {
   require(cs.size() == gs.size() && !cs.empty(), GB200_ERR_INVALID, "split group: one contraction per context");
@@ -1405,7 +1481,7 @@ void split_gemm_group(const std::vector<Context*>& cs, const std::vector<ZGemm>&
   std::vector<SplitEngine*> ses;
   std::vector<int> bns;
   int64_t nch = 0;
-  bool tc_engine = true;
+  bool tc_engine = true, overlap = true;
   for (size_t i = 0; i < cs.size(); ++i) {
     for (size_t j = 0; j < i; ++j)
       require(cs[j] != cs[i], GB200_ERR_INVALID, "split group: a context appears twice (its slice buffers are shared)");
@@ -1413,13 +1489,14 @@ void split_gemm_group(const std::vector<Context*>& cs, const std::vector<ZGemm>&
     require(gs[i].K > 0 && gs[i].M > 0 && gs[i].N > 0, GB200_ERR_INVALID, "split group: empty contraction");
     ses.push_back(split_engine(*cs[i]));
     tc_engine = tc_engine && ses.back()->core == 0;
-    bns.push_back(tile_width(*cs[i], S, gs[i].N));
+    overlap = overlap && overlap_mode(S, gs[i].K);
     nch = std::max<int64_t>(nch, (gs[i].K + kmax - 1) / kmax);
   }
   if (!tc_engine) {  // the CUDA-core validation engine has no grouped form
     for (size_t i = 0; i < cs.size(); ++i) split_gemm(*cs[i], *ses[i], gs[i], st, S);
     return;
   }
+  for (size_t i = 0; i < cs.size(); ++i) bns.push_back(tile_width(*cs[i], S, gs[i].M, overlap));
   SplitEngine& se0 = *ses[0];
   // K chunk ch of every problem that has one, all in one grouped launch per chunk
   for (int64_t ch = 0; ch < nch; ++ch) {
@@ -1427,25 +1504,24 @@ void split_gemm_group(const std::vector<Context*>& cs, const std::vector<ZGemm>&
     int BNmax = 16;
     double flops = 0.0;
     int64_t total = 0;
-    bool sink = false;
     for (size_t i = 0; i < cs.size(); ++i) {
       const int64_t k0 = ch * kmax;
       if (k0 >= gs[i].K) continue;
       Prepared pr = prepare_chunk(*ses[i], gs[i], S, bns[i], k0, std::min(kmax, gs[i].K - k0), st);
       GroupEntry e;
-      e.mA = pr.mA;
-      e.mB = pr.mB;
+      e.mR = pr.mR;
+      e.mC = pr.mC;
       e.p = pr.p;
       e.tile_begin = total;
       entries.push_back(e);
       total += pr.ntiles;
       BNmax = std::max(BNmax, bns[i]);
       flops += pr.flops;
-      sink = sink || pr.p.sink.expo != nullptr;
     }
     GemmParams p{};
     p.S = S;
     p.BN = BNmax;
+    p.overlap = overlap ? 1 : 0;
     p.err = se0.err.p;
     size_t smem = 0;
     ring_layout(S, BNmax, p, smem);
@@ -1455,7 +1531,7 @@ void split_gemm_group(const std::vector<Context*>& cs, const std::vector<ZGemm>&
     p.ngroup = (int)entries.size();
     p.ntiles = total;
     KernelRecord* rec = begin_record(*cs[0], flops, st);
-    launch_tc<true>(S, sink, persistent_grid(*cs[0], total), smem, st, entries[0].mA, entries[0].mB, p);
+    launch_tc<true>(S, persistent_grid(*cs[0], total), smem, st, entries[0].mR, entries[0].mC, p);
     if (rec) GB_CUDA(cudaEventRecord(rec->stop, st));
   }
 }

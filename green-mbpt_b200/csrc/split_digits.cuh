@@ -1,6 +1,13 @@
-// Balanced base-128 digits of the split-precision slices (shared by the slicer kernels and the
-// host-side test of the digit arithmetic).
+// Balanced digits of the split-precision slices (shared by the slicer kernels and the host-side test of the
+// digit arithmetic): base 256 for up to six slices, base 128 for seven and eight (whose base-256 form would
+// exceed the 53 bits of the operand).
 //
+// Base 256.  With the row exponent e (|a| < 2^(e-1)) and X = rint(a 2^(8S - 1 - e)), |X| <= 2^(8S-2) and
+// X = sum_p d_p 256^p with d_p in [-128, 127] (|d| <= 64 for the top one).  Adding 128 in every digit turns them into
+// the bytes of X + H, H = 128 (256^S - 1) / 255, so digit p is that byte with its top bit flipped.  The same count of
+// slices and digit products holds four bits more at S = 5 than base 128, whose digits use half of the INT8 range.
+//
+// Base 128.
 // With the row exponent e (|a| < 2^(e-1)) and X = rint(a 2^(7S - e)), |X| < 2^(7S-1) and
 // X = sum_p d_p 128^p with d_p in [-64, 63] for p < S - 1 and the top digit in [-64, 64].
 // Rounding to nearest and signed digits make both the representation error and the digit products
@@ -70,6 +77,36 @@ GB_DIGITS_FN uint32_t balanced_digit_word(uint64_t u0, uint64_t u1, uint64_t u2,
 #endif
   if (s > 0) w &= 0x7F7F7F7Fu;  // the top digit takes all bits above it (at most 128)
   return w ^ 0x40404040u ^ ((~w & 0x40404040u) << 1);
+}
+
+// X + H for X = rint(x), |x| <= 2^(8S-2), S <= 6: 1.5 * 2^52 leaves rint(x) in the low mantissa bits of the sum.
+// Only the low 8 S bits of the result mean anything.  wide_negate gives the same of -X.
+GB_DIGITS_FN uint64_t wide_bias(int S) { return ((((uint64_t)1) << (8 * S)) - 1) / 255 * 128; }
+GB_DIGITS_FN uint64_t wide_input(double x, int S) {
+  const double t = x + 6755399441055744.0;
+#ifdef __CUDA_ARCH__
+  const uint64_t bits = (uint64_t)__double_as_longlong(t);
+#else
+  uint64_t bits;
+  std::memcpy(&bits, &t, sizeof bits);
+#endif
+  return bits - 0x4338000000000000ull + wide_bias(S);
+}
+GB_DIGITS_FN uint64_t wide_negate(uint64_t u, int S) { return 2 * wide_bias(S) - u; }
+
+// Digit s (s = 0 the top one) of four values: byte i of the word is that of U_i.
+GB_DIGITS_FN uint32_t wide_digit_word(uint64_t u0, uint64_t u1, uint64_t u2, uint64_t u3, int S, int s) {
+  const int p = S - 1 - s;
+#ifdef __CUDA_ARCH__
+  const int sel = p & 3, pick = sel | ((4 + sel) << 4);
+  const uint32_t t0 = (uint32_t)(p < 4 ? u0 : u0 >> 32), t1 = (uint32_t)(p < 4 ? u1 : u1 >> 32),
+                 t2 = (uint32_t)(p < 4 ? u2 : u2 >> 32), t3 = (uint32_t)(p < 4 ? u3 : u3 >> 32);
+  return __byte_perm(__byte_perm(t0, t1, pick), __byte_perm(t2, t3, pick), 0x5410) ^ 0x80808080u;
+#else
+  const uint32_t w = (uint32_t)((u0 >> (8 * p)) & 0xFFu) | (uint32_t)((u1 >> (8 * p)) & 0xFFu) << 8 |
+                     (uint32_t)((u2 >> (8 * p)) & 0xFFu) << 16 | (uint32_t)((u3 >> (8 * p)) & 0xFFu) << 24;
+  return w ^ 0x80808080u;
+#endif
 }
 
 // two's complement negation of each byte (no carry between bytes)

@@ -4,18 +4,19 @@ Test infrastructure, like gw_oracle.py: nothing in the product imports it.  It r
 arithmetic of the library's split engine in numpy:
 - a per-row exponent for the left operand and a per-column exponent for the right one, taken
   over the contraction range, with one bit of headroom (max of |Re| and |Im| < 2^(e-1));
-- rounding X = rint(a 2^(7S - e)) and its S balanced base-128 digits;
+- rounding to an integer of S balanced base-256 digits (base 128 above six slices);
 - the digit products of the diagonals i + j <= S - 1, summed exactly.
 The engine's first form (truncation toward zero, sign-magnitude digits) is kept as
 digits="truncated" for comparison.
 `gw_split_model` runs the six contractions of the GPU's GW pipeline with the same operand roles:
-P0 (a) T1^T = G^T V^T, (b) Bt = Gbar T1, (c) P0^T = conj(V) Bt^T; Sigma (d) Y1^T = G^T V^T,
-(e) Y2^T = W^T Y1, (f) Sigma^T = conj(V) Y2^T.  Each takes its own slice count, or FP64.  The W
-solve and the transforms are FP64, as on the GPU.
+P0 (a) T1^T = G^T V^T, (b) Bt = Gbar T1, (c) P0^T = conj(V) Bt^T; Sigma (d) X = G V^H,
+(e) Z = V^T W, (f) Sigma = Z X (or, without mirror symmetry and spin, (d) Y1^T = G^T V^T, (e) Y2^T = W^T Y1,
+(f) Sigma^T = conj(V) Y2^T).  Each takes its own slice count, or FP64.  The W solve and the transforms are FP64, as on
+the GPU.
 
 For one iteration from G0 on a c2-shaped system (nao=40, naux=250, ntau=120, nw=120, beta=200,
 eps ~ U[-5,5], 2x1x1 mesh, seed 0), five slices everywhere: the truncated form gives
-max|dSigma| = 1.0344e-7, as the GPU measured with it (1.0344e-7); the balanced form gives 3.1e-9.
+max|dSigma| = 1.0344e-7, as the GPU measured with it (1.0344e-7); balanced base-128 digits gave 3.1e-9.
 Truncation toward zero biases every digit product the same way, so its errors add in phase along
 each contraction and across the six of them.
 
@@ -36,54 +37,57 @@ CONTRACTIONS = "abcdef"
 def split_mm(A, B, S, digits="balanced"):
     """A (M,K) @ B (K,N), complex, as the split engine forms it.  Exponents: per row of A and per
     column of B, over K, of max(|Re|, |Im|).
-    - "balanced" (the engine): e = frexp exponent + 1, X = rint(a 2^(7S-e)), balanced base-128 digits
-      (lower ones in [-64, 63], the top one the remaining quotient);
-    - "truncated" (the engine's first form): e = frexp exponent, X = trunc(a 2^(7S-e)), digits of |X|
+    - "balanced" (the engine): e = frexp exponent + 1; up to six slices X = rint(a 2^(8S-1-e)) in balanced base-256
+      digits (lower ones in [-128, 127], the top one the remaining quotient), for more X = rint(a 2^(7S-e)) in
+      base-128 ones ([-64, 63]);
+    - "truncated" (the engine's first form): e = frexp exponent, X = trunc(a 2^(7S-e)), base-128 digits of |X|
       carrying the sign of a.
-    Digit products of the diagonals i + j <= S - 1 are kept; S = None is the FP64 product."""
+    -Im A is cut into digits of its own (the negative of a digit -128 is none).  Digit products of the diagonals
+    i + j <= S - 1 are kept; S = None is the FP64 product."""
     if S is None:
         return A @ B
     bal = digits == "balanced"
+    bits = 8 if bal and S <= 6 else 7
+    base, half = 2 ** bits, 2 ** (bits - 1)
 
     def expo(X, axis):
         m = np.maximum(np.abs(X.real), np.abs(X.imag)).max(axis=axis)
         _, e = np.frexp(m)
         return np.where(m > 0, e + (1 if bal else 0), 0)
 
-    def planes_of(X, e, rows):
-        sc = np.ldexp(1.0, 7 * S - e)
+    def planes_of(part, e, rows):
+        sc = np.ldexp(1.0, bits * S - (bits - 7) - e)
         sc = sc[:, None] if rows else sc[None, :]
-        out = []
-        for part in (X.real, X.imag):
-            if bal:
-                Xi = np.rint(part * sc)
-                planes = [None] * S
-                for i in range(S - 1, 0, -1):
-                    d = np.mod(Xi + 64, 128) - 64
-                    planes[i] = d
-                    Xi = (Xi - d) / 128
-                planes[0] = Xi
-            else:
-                Xi = np.trunc(part * sc)
-                mag, sg = np.abs(Xi), np.sign(Xi)
-                planes = [sg * (np.floor(mag / 2.0 ** (7 * (S - 1 - i))) % 128) for i in range(S)]
-            out.append(planes)
-        return [out[0][i] + 1j * out[1][i] for i in range(S)]
+        if bal:
+            Xi = np.rint(part * sc)
+            planes = [None] * S
+            for i in range(S - 1, 0, -1):
+                d = np.mod(Xi + half, base) - half
+                planes[i] = d
+                Xi = (Xi - d) / base
+            planes[0] = Xi
+            return planes
+        Xi = np.trunc(part * sc)
+        mag, sg = np.abs(Xi), np.sign(Xi)
+        return [sg * (np.floor(mag / 2.0 ** (7 * (S - 1 - i))) % 128) for i in range(S)]
 
     eA, eB = expo(A, 1), expo(B, 0)
-    dA, dB = planes_of(A, eA, True), planes_of(B, eB, False)
+    ar, ai, an = (planes_of(x, eA, True) for x in (A.real, A.imag, -A.imag))
+    br, bi = (planes_of(x, eB, False) for x in (B.real, B.imag))
     C = np.zeros((A.shape[0], B.shape[1]), dtype=np.complex128)
     for d in range(S):
         acc = np.zeros_like(C)
         for i in range(d + 1):
-            acc += dA[i] @ dB[d - i]
-        C += np.ldexp(1.0, -7 * (d + 2)) * acc
+            acc.real += ar[i] @ br[d - i] + an[i] @ bi[d - i]
+            acc.imag += ai[i] @ br[d - i] + ar[i] @ bi[d - i]
+        C += np.ldexp(1.0, -14 - bits * d) * acc
     return C * np.ldexp(1.0, eA)[:, None] * np.ldexp(1.0, eB)[None, :]
 
 
-def gw_split_model(s, Sc, digits="balanced"):
+def gw_split_model(s, Sc, digits="balanced", by_z=True):
     """Sigma(tau, k) of the synthetic system `s` with contraction c in 'abcdef' run at Sc[c] slices
-    (None: FP64), digits as in split_mm."""
+    (None: FP64), digits as in split_mm.  by_z: Sigma through X = G V^H and Z = V W (two spins or mirror
+    symmetric transforms), else through Y1 = V G and Y2 = Y1^T W."""
     g = s.grid
     integ, bz = O.HalfStoredIntegrals(s.V_half), O.NoSymBZ(s.mesh)
     G = s.G
@@ -137,6 +141,19 @@ def gw_split_model(s, Sc, digits="balanced"):
             kmq = bz.k2_from_k1q(k, q)
             V = integ.pair(k, kmq)                          # [Q][i][m]
             Gm = G[:, :, kmq]                               # [t][s][m][n]
+            if by_z:
+                # (d) X[(t,s,m)][(Q',j)] = sum_n Gm[t,s][m][n] conj(V[Q'][j][n])
+                X = split_mm(Gm.reshape(nts * ns * nao, nao), np.conj(V).reshape(NQ * nao, nao).T, Sc["d"], digits)
+                X = X.reshape(nts, ns, nao, NQ, nao)                           # [t][s][m][Q'][j]
+                for t in range(nts):
+                    # (e) Z[(i,m)][Q'] = sum_Q V[Q][(i,m)] W[t][Q][Q']
+                    Z = split_mm(V.reshape(NQ, nao * nao).T, W[t], Sc["e"], digits).reshape(nao, nao, NQ)
+                    # (f) Sigma[i][(s,j)] = -sum_{(m,Q')} Z[i][(m,Q')] X[s][(m,Q')][j]
+                    A = Z.reshape(nao, nao * NQ)
+                    B = np.transpose(X[t], (1, 2, 0, 3)).reshape(nao * NQ, ns * nao)
+                    R = split_mm(A, B, Sc["f"], digits).reshape(nao, ns, nao)
+                    Sig[t, :, k] -= np.transpose(R, (1, 0, 2))
+                continue
             # (d) Y1^T[(t,s,n)][(Q,i)] = sum_m Gm[t,s][m][n] V[Q][i][m]
             A = np.transpose(Gm, (0, 1, 3, 2)).reshape(nts * ns * nao, nao)
             B = np.transpose(V, (2, 0, 1)).reshape(nao, NQ * nao)
