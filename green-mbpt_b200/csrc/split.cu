@@ -70,21 +70,26 @@ __device__ __forceinline__ void mbar_arrive_local(uint64_t* bar) {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
+// The time hint lets the hardware keep the thread asleep instead of polling: without it the waiting warps issued a third
+// of the SM's instructions, in competition with the warps they waited for.
+constexpr uint32_t WAIT_HINT_NS = 20000;
+
 __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t phase) {
   uint32_t ok;
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
-      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+      "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
       "selp.u32 %0, 1, 0, p;\n\t}"
       : "=r"(ok)
-      : "r"(smem_u32(bar)), "r"(phase)
+      : "r"(smem_u32(bar)), "r"(phase), "r"(WAIT_HINT_NS)
       : "memory");
   return ok != 0;
 }
 
 // Bounded wait: returns false on timeout.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
-  long long t0 = clock64();
+  if (mbar_try_wait(bar, phase)) return true;
+  const long long t0 = clock64();
   while (!mbar_try_wait(bar, phase)) {
     if (*abort_flag) return false;
     if (clock64() - t0 > WAIT_LIMIT) return false;
@@ -887,15 +892,19 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
       }
     }
   } else if (warp == 2) {
+    // (this warp works beside four busy epilogue warps, so it keeps to what changes: the problem's constants are written
+    // once per set, and 32-bit indices serve wherever a tile's share allows)
     uint32_t tcount = 0, nr = 0;  // tiles, row tables written (the last in set (nr - 1) & 1)
+    const GemmParams* head_q[2] = {nullptr, nullptr};
     for (TileWalk<GROUPED> w(p, &mapR, &mapC, t_first, t_end, t_step); w.more(); w.next(), ++tcount) {
       const int set = (int)(tcount & 1);
       const GemmParams& q = *w.q;
-      const int64_t row0 = w.row0(), m0 = w.col0() / 2;
-      const int64_t rlim = q.N - row0, clim = q.M - m0;
+      const int64_t row0 = w.row0(), m0 = w.col0() >> 1;
+      const int half = q.BN >> 1;
+      const int rlim = (int)(q.N - row0 < TILE_R ? q.N - row0 : TILE_R), clim = (int)(q.M - m0 < half ? q.M - m0 : half);
       // this tile's exponents are on their way while the table set is waited for
       const int32_t* eA = q.eA + w.rbA * q.eA_ld + m0;
-      const bool cin = lane < clim && lane < q.BN / 2;
+      const bool cin = lane < clim;
       const int e0 = cin ? eA[lane] : 0;
       const int64_t o0 = cin ? q.C.row(m0 + lane) : 0;
       bool ok = true;
@@ -909,7 +918,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
       }
       uint8_t* tb = tables + set * tsb;
       int64_t* coff = reinterpret_cast<int64_t*>(tb + sizeof(TileHead));
-      double* csc = reinterpret_cast<double*>(coff + q.BN / 2);
+      double* csc = reinterpret_cast<double*>(coff + half);
       if (w.new_rows) {
         // new rows go to the other row set; its last tile lies at least two tiles back and has been stored
         int64_t* roff = reinterpret_cast<int64_t*>(row_tables + (nr & 1) * ROW_TABLE_BYTES);
@@ -929,11 +938,11 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
           rsc[i] = pow2(e[j]) * al;
         }
       }
-      if (lane < q.BN / 2) {
+      if (lane < half) {
         coff[lane] = o0;
         csc[lane] = pow2(e0 - unit_exp(S));
       }
-      for (int i = lane + 32; i < q.BN / 2; i += 32) {
+      for (int i = lane + 32; i < half; i += 32) {
         const bool in = i < clim;
         coff[i] = in ? q.C.row(m0 + i) : 0;
         csc[i] = pow2((in ? eA[i] : 0) - unit_exp(S));
@@ -941,16 +950,19 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
       if (lane == 0) {
         TileHead& h = *reinterpret_cast<TileHead*>(tb);
         h.C = q.C.ptr + q.C.bat(w.b0, w.b1, w.b2);
-        h.rlim = (int)(rlim < TILE_R ? rlim : TILE_R);
-        h.clim = (int)(clim < q.BN / 2 ? clim : q.BN / 2);
-        h.ngroups = (2 * h.clim + EPI_CG - 1) / EPI_CG;
-        h.bn = q.BN;
+        h.rlim = rlim;
+        h.clim = clim;
+        h.ngroups = (2 * clim + EPI_CG - 1) / EPI_CG;
         h.rowset = (int)((nr - 1) & 1);
-        h.scaled = !q.alpha_pow2;
-        h.has_beta = q.beta.x != 0.0 || q.beta.y != 0.0;
-        h.alpha = q.alpha;
-        h.beta = q.beta;
+        if (head_q[set] != w.q) {
+          h.bn = q.BN;
+          h.scaled = !q.alpha_pow2;
+          h.has_beta = q.beta.x != 0.0 || q.beta.y != 0.0;
+          h.alpha = q.alpha;
+          h.beta = q.beta;
+        }
       }
+      head_q[set] = w.q;
       __syncwarp();
       if (lane == 0) mbar_arrive_local(&tabf_bar[set]);
     }
