@@ -9,11 +9,12 @@
 // one barrier per block.  K-fastest operands are kept [row][k] with 4 spare elements a row, the others [k][row]
 // with 2 spare, so that the 8 lanes of a 128-bit fragment read hit different banks in both.
 //
-// Two CTAs of 128 threads share an SM (up to 255 registers a thread): one of them stores its tile or fills its
-// ring while the other multiplies.  What bounds it is the FP64 tensor pipe (37 TFLOP/s from registers): 71 % of it
+// Two or three CTAs of 128 threads share an SM (255 or 168 registers a thread): one of them stores its tile or fills
+// its ring while another multiplies (three instead of two for the smaller tiles: 10.0 -> 9.0 ms on the exchange below,
+// 132 -> 122 ms on a two-spin self-energy at nao = 26).  What bounds it is the FP64 tensor pipe (37 TFLOP/s from registers): 71 % of it
 // on 150 x 150 x 10816, half on contractions as short as K = 26, where the index maps and the stores count.  Copies
 // issued between the products instead of before them were slower (their address loads stall the warp that multiplies).
-// Exchange of a Fock build at nk = 27, nao = 40, NQ = 250: 29.4 -> 10.0 ms against the 64 x 64 kernel with register
+// Exchange of a Fock build at nk = 27, nao = 40, NQ = 250: 29.4 -> 9.0 ms against the 64 x 64 kernel with register
 // staging that this one replaced.
 // Contractions with few tiles split K over a cluster of up to 8 CTAs and sum the parts through distributed
 // shared memory in rank order, so a result never depends on timing.
@@ -42,7 +43,9 @@ struct Tile {
   static constexpr int BK = WK == 1 ? 8 : 16;
   static constexpr int A_ELEMS = MT * (BK + 4), B_ELEMS = NTL * (BK + 4);  // [k][row] needs no more: BK <= 2 rows
   static constexpr int STAGE = A_ELEMS + B_ELEMS;
-  static constexpr int RING_MAX = 106 * 1024 / (STAGE * 16);
+  // CTAs of an SM: three where the warp's accumulators leave the registers for it (170 a thread)
+  static constexpr int CTAS = TM * TN <= 10 ? 3 : 2;
+  static constexpr int RING_MAX = (CTAS == 3 ? 70 : 106) * 1024 / (STAGE * 16);
   static constexpr int STAGES = RING_MAX > 4 ? 4 : RING_MAX;
   static constexpr int RED = (WK * MT * NTL);  // elements of the partial sums (reuses the ring)
   static constexpr size_t SMEM = (size_t)(STAGES * STAGE > RED ? STAGES * STAGE : RED) * sizeof(cplx);
@@ -99,7 +102,7 @@ __device__ __forceinline__ void load_block(cplx* s, const cplx* base, const IdxM
 }
 
 template <int TM, int TN, int WN>
-__global__ void __launch_bounds__(NT, 2)
+__global__ void __launch_bounds__(NT, (Tile<TM, TN, WN>::CTAS))
     zgemm_fp64_kernel(const __grid_constant__ ZGemm g, LoadMode lm, int64_t nbatch, int ksplit) {
   using T = Tile<TM, TN, WN>;
   constexpr int BK = T::BK;
