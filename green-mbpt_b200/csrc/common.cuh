@@ -124,6 +124,9 @@ struct ZGemm {
 };
 
 void zgemm_fp64(const ZGemm& g, cudaStream_t st);
+// Load every tile variant's code on the current device now (it is otherwise loaded, into device memory, at its first
+// use): for callers that must not allocate later or will be captured.
+void zgemm_fp64_preload();
 void validate(const ZGemm& g);
 void set_thread_error(const std::string& msg);
 

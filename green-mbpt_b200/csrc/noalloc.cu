@@ -84,6 +84,8 @@ void* scratch_address(int dev, cudaStream_t st) {
             "hf_fock_noalloc: the first call in this context must come before stream capture");
     return ent.ptr;
   }
+  // a later call may need another tile variant of the GEMM; all of them are loaded with the first one
+  if (ent.ctx != cur) zgemm_fp64_preload();
   ent.ctx = cur;
   ent.ptr = p;
   return p;

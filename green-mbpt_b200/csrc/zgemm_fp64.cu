@@ -326,7 +326,34 @@ void launch_tm(int tm, const ZGemm& g, const LoadMode& lm, int64_t nbatch, int k
   }
 }
 
+template <int TN, int WN, int TM>
+void preload_one() {
+  if constexpr (TM * TN <= 16) {
+    cudaFuncAttributes at;
+    GB_CUDA(cudaFuncGetAttributes(&at, zgemm_fp64_kernel<TM, TN, WN>));
+  }
+}
+
+template <int TN, int WN>
+void preload_tn() {
+  preload_one<TN, WN, 1>();
+  preload_one<TN, WN, 2>();
+  preload_one<TN, WN, 3>();
+  preload_one<TN, WN, 4>();
+  preload_one<TN, WN, 5>();
+  preload_one<TN, WN, 6>();
+  preload_one<TN, WN, 7>();
+  preload_one<TN, WN, 8>();
+}
+
 }  // namespace
+
+void zgemm_fp64_preload() {
+  preload_tn<2, 4>();
+  preload_tn<3, 2>();
+  preload_tn<2, 2>();
+  preload_tn<2, 1>();
+}
 
 void validate(const ZGemm& g) {
   // an outer index with neither a table nor a stride is a set-up error, not a broadcast
