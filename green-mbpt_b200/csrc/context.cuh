@@ -105,11 +105,12 @@ struct Context {
   struct WTransforms {
     int nu = 0;            // frequencies
     int nt = 0;            // times of W: nts, or nts / 2 with W(beta - tau) = W(tau)
-    DevArray<cplx> fwd;    // [nu][nts / 2]
-    DevArray<cplx> bwd;    // [nt][nu]
+    const cplx* fwd = nullptr;  // [nu][nts / 2]
+    const cplx* bwd = nullptr;  // [nt][nu]
     std::vector<cplx> bwd_host;  // [nts][nu]
   };
   WTransforms w_exact, w_mirror;  // w_mirror.nu = 0: the grid has no such symmetry
+  DevArray<cplx> w_tables;        // their matrices; w_exact.bwd is Ttn_b itself
   DevArray<int64_t> tab_x_mirror; // rows (t, s) of X in mirror-pair order: element offset of (t, s)
   // q -> 0 correction ("extrapolate" treatment, mbpt_q0_utils_t): AqQ [nk][NQ] on the device,
   // |q| on the host, the Madelung constant; eps_inv [nw_b][nk] collects the heads of P(i Omega, q)

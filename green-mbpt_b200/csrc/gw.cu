@@ -201,8 +201,6 @@ void build_w_transforms(Context& c, const cplx* Tnt, const cplx* Ttn) {
   Context::WTransforms& e = c.w_exact;
   e.nu = nw;
   e.nt = nts;
-  e.fwd.upload(fold.data(), fold.size(), c.stream);
-  e.bwd.upload(Ttn, (size_t)nts * nw, c.stream);
   e.bwd_host.assign(Ttn, Ttn + (size_t)nts * nw);
   // frequencies with equal folded rows (each joins the first such one)
   std::vector<int> group(nw, -1), first;
@@ -250,16 +248,22 @@ void build_w_transforms(Context& c, const cplx* Tnt, const cplx* Ttn) {
   m.nu = finite && asym <= MIRROR_TOL * bmax ? nu : 0;
   if (m.nu > 0) {
     m.nt = nth;
-    m.fwd.upload(fwd.data(), fwd.size(), c.stream);
-    m.bwd.upload(half.data(), half.size(), c.stream);
     m.bwd_host = full;
+    fold.insert(fold.end(), fwd.begin(), fwd.end());
+    fold.insert(fold.end(), half.begin(), half.end());
     std::vector<int64_t> tab((size_t)nts * ns);
     for (int t = 0; t < nts; ++t)
       for (int s = 0; s < ns; ++s)
         tab[(size_t)t * ns + s] = ((int64_t)(t < nth ? 2 * t : 2 * (nts - 1 - t) + 1) * ns + s) * c.pair_elems();
     c.tab_x_mirror.upload(tab.data(), tab.size(), c.stream);
+    GB_CUDA(cudaStreamSynchronize(c.stream));
   }
+  c.w_tables.upload(fold.data(), fold.size(), c.stream);
   GB_CUDA(cudaStreamSynchronize(c.stream));
+  e.fwd = c.w_tables.get();
+  e.bwd = c.Ttn_b.get();
+  m.fwd = e.fwd + (size_t)nw * nth;
+  m.bwd = m.fwd + fwd.size();
 }
 
 // Choose the k-block size so that the intermediates (and, without a caller's budget, the slice planes of the largest
@@ -526,7 +530,7 @@ struct GwRun {
     {
       ZGemm f;  // Pw[n] = sum_t Tnt_b[n][t] P0[t]
       f.M = nu; f.N = (int64_t)NQ * NQ; f.K = nth;
-      f.A = dense(wt->fwd.get(), nth);
+      f.A = dense(wt->fwd, nth);
       f.B = dense(P0, (int64_t)NQ * NQ);
       f.C.ptr = Pw; f.C.row = lin((int64_t)NQ * NQ); f.C.col = lin(1);
       zgemm_fp64(f, st);
@@ -559,7 +563,7 @@ struct GwRun {
       }
       ZGemm bt;  // W(tau) = sum_n Ttn_b[t][n] P(i Omega_n) -> stored in P0
       bt.M = ntz; bt.N = (int64_t)NQ * NQ; bt.K = nu;
-      bt.A = dense(wt->bwd.get(), nu);
+      bt.A = dense(wt->bwd, nu);
       bt.B = dense(aug, (int64_t)NQ * NQ);
       bt.C.ptr = P0; bt.C.row = lin((int64_t)NQ * NQ); bt.C.col = lin(1);
       zgemm_fp64(bt, st);
