@@ -77,10 +77,10 @@ __device__ int pivot_search(const cplx* aug, int64_t ld, int j, int n, double* s
 // holds the elements (ti + TI a, tj + 16 b).  Step k publishes column k and the scaled pivot row in shared memory and
 // every thread updates its elements from them; rows stay where they are and the pivot order is undone when the result
 // is stored.  The block of 16 columns that k lies in is a compile-time index, and column k and the pivot row are
-// cleared by their holders, so the update is 4 RI CJ multiply-adds and nothing else.  PIVOT: partial pivoting (every
+// cleared by their holders, so the update is 6 RI CJ FP64 operations and nothing else.  PIVOT: partial pivoting (every
 // warp finds the largest unused element of the column by itself, two barriers a step); otherwise the diagonal in order,
 // one barrier a step, and a pivot that is not positive is reported.
-// Against the augmented matrix in shared memory that it replaced, 15000 matrices of n = 40: 4.96 -> 1.0 ms, with the
+// Against the augmented matrix in shared memory that it replaced, 15000 matrices of n = 40: 4.96 -> 1.13 ms, with the
 // assembly of the matrices and the trace in the same pass (0.12 + 0.55 ms before).
 // Many matrices (the Dyson step): 128 threads each, five of them on an SM, which cover one another's barriers and
 // pivot searches.  Few matrices (the screened interaction): 256 threads each, because only the latency counts.
@@ -186,9 +186,11 @@ __device__ __forceinline__ bool gj_invert(cplx (&m)[RI][CJ], int n, GjShared& sh
         if (ti + TI * a == p) f = cmk(-1.0, 0.0);
 #pragma unroll
         for (int b = 0; b < CJ; ++b) {
+          // the product first, then one subtraction: an element much larger than the product is rounded once (two
+          // chained FMAs: 1.0 ms instead of 1.13, but an error of 2.4e-15 where the augmented form had 2.0e-15)
           cplx& e = m[a][b];
-          e.x = fma(f.y, r[b].y, fma(-f.x, r[b].x, e.x));
-          e.y = fma(-f.y, r[b].x, fma(-f.x, r[b].y, e.y));
+          e.x += fma(-f.x, r[b].x, f.y * r[b].y);
+          e.y -= fma(f.x, r[b].y, f.y * r[b].x);
         }
       }
     }
