@@ -41,8 +41,9 @@ import numpy as np  # noqa: E402
 
 METRIC = "GW iterations/s at nk=125,nao=40: split-prec vs FP64 on B200, max|ΔΣ|≤1e-8"
 # DRAM bytes (read + write) per FP64-equivalent flop of the tensor-core contraction kernel, from
-# one ncu capture of its six launch shapes on the c2-shaped profiling case (c2k2) with the current
-# kernel (profiles/split_gemm_tc_c2k2.md): 8.25 GB for 3.80e11 flops.  Each shape's traffic scales
+# one ncu capture of its six launch shapes on the c2-shaped profiling case (c2k2) with an earlier
+# form of the kernel (profiles/split_gemm_tc_c2k2.md): 8.25 GB for 3.80e11 flops; (a) to (d) of the current
+# kernel move 4.27 GB where that form moved 4.51.  Each shape's traffic scales
 # with its k-point batch as its flops do, so the roofline traffic per launch is this ratio times
 # the step's flops per launch.
 TC_DRAM_BYTES_PER_FLOP = 8.25e9 / 3.80e11
@@ -435,7 +436,7 @@ def main_ours(args):
         line = {
             "metric": METRIC, "value": 1.0 / comp_s, "unit": UNIT, "n_gpus": ws, "steps": K, "warmup": args.warmup,
             "ms_per_step": comp_s * 1e3, "higher_is_better": True, "scaling": "strong", "vs_baseline": None,
-            "dtype": (f"int8 ({args.slices} balanced base-128 slices per FP64 operand, int32 tensor-core "
+            "dtype": (f"int8 ({args.slices} balanced base-256 slices per FP64 operand (base 128 above six), int32 tensor-core "
                       "accumulate, f64 recombination; f64 aux-basis solve, transforms, Dyson)"),
             "data": "synthetic (seeded generator; V generated on the GPU)",
             "config": {"workload": WORKLOADS[args.config],
