@@ -97,6 +97,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, volatil
   return true;
 }
 
+// The whole warp waits, one lane polls.  The shuffle brings the other lanes the outcome but orders no memory; __syncwarp
+// is what carries the polling lane's acquire over to their reads and writes.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
+  int ok = 1;
+  if (threadIdx.x % 32 == 0) ok = mbar_wait(bar, phase, abort_flag);
+  __syncwarp();
+  return __shfl_sync(0xffffffffu, ok, 0) != 0;
+}
+
 __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
   asm volatile(
       "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(
@@ -907,9 +916,7 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
       const bool cin = lane < clim;
       const int e0 = cin ? eA[lane] : 0;
       const int64_t o0 = cin ? q.C.row(m0 + lane) : 0;
-      bool ok = true;
-      if (lane == 0) ok = mbar_wait(&tabe_bar[set], ((tcount >> 1) & 1) ^ 1, abort_flag);
-      if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) {
+      if (!mbar_wait_warp(&tabe_bar[set], ((tcount >> 1) & 1) ^ 1, abort_flag)) {
         if (lane == 0) {
           atomicExch(p.err, SERR_TIMEOUT_TABLES);
           *abort_flag = 1;
@@ -975,10 +982,8 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
     int buf = 0;
     for (uint32_t t = t_first; t < t_end; t += t_step, ++tcount) {
       const int set = (int)(tcount & 1);
-      bool ok = true;
-      if (lane == 0)
-        ok = mbar_wait(&tabf_bar[set], (tcount >> 1) & 1, abort_flag) && mbar_wait(&accf_bar[buf], acc_ph, abort_flag);
-      if (!__shfl_sync(0xffffffffu, ok ? 1 : 0, 0)) {
+      if (!mbar_wait_warp(&tabf_bar[set], (tcount >> 1) & 1, abort_flag) ||
+          !mbar_wait_warp(&accf_bar[buf], acc_ph, abort_flag)) {
         if (lane == 0) {
           atomicExch(p.err, SERR_TIMEOUT_EPILOGUE);
           *abort_flag = 1;
