@@ -100,8 +100,8 @@ struct Context {
   std::vector<cplx> Ttn_beta;  // host copy of the tau = beta row of Ttn_f
   // The bosonic transforms as the q loop applies them.  P0(tau) is mirrored exactly (P0(beta - tau) = P0(tau)), so the
   // forward one is folded onto the first half of tau.  `exact` keeps every frequency and time.  `mirror` also merges
-  // frequencies whose folded rows agree (+-Omega) and gives W on the first half of tau only: usable when the given
-  // matrices are mirror symmetric to well below a contraction's slice rounding (build_w_transforms).
+  // frequencies whose folded rows agree (+-Omega) and gives W on the first half of tau only: usable when that changes W
+  // by less than a contraction's slice rounding (w_transforms.h).
   struct WTransforms {
     int nu = 0;            // frequencies
     int nt = 0;            // times of W: nts, or nts / 2 with W(beta - tau) = W(tau)

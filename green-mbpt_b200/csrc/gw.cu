@@ -16,11 +16,13 @@
 //      Sigma: Y1 = V G(tau,k-q);  Y2 = Y1^T W(tau);           Sigma -= Y2 . conj(V).
 #include <algorithm>
 #include <cmath>
+#include <complex>
 #include <memory>
 #include <vector>
 
 #include "context.cuh"
 #include "split.cuh"
+#include "w_transforms.h"
 
 namespace gb200 {
 namespace {
@@ -182,75 +184,31 @@ void build_subset_tables(Context& c) {
   GB_CUDA(cudaStreamSynchronize(c.stream));
 }
 
-// The largest mirror asymmetry of the transforms, relative to their largest element, at which the folded form is used:
-// 2^-39, the unit in which five slices hold an operand.  (The synthetic Chebyshev grids have
-// 1e-13 to 5e-13, so FP64 and six slices keep the matrices as given.)
-constexpr double MIRROR_TOL = 1.8e-12;
+// Slice counts up to which W may be taken through the mirror-symmetric form (w_transforms.h): the form's change stays
+// below what five slices resolve; six slices and FP64 apply the matrices as given.
 constexpr int MIRROR_MAX_SLICES = 5;
 
 void build_w_transforms(Context& c, const cplx* Tnt, const cplx* Ttn) {
   const int nts = c.d.nts, nth = nts / 2, nw = c.d.nw_b, ns = c.ns_eff();
-  std::vector<cplx> fold((size_t)nw * nth);
-  double fmax = 0.0, bmax = 0.0;
+  using host_cplx = std::complex<double>;
+  std::vector<cplx> tables((size_t)nw * nth);  // the folded forward transform, then the merged and the mirrored ones
   for (int n = 0; n < nw; ++n)
-    for (int t = 0; t < nth; ++t) {
-      const cplx v = cadd(Tnt[(size_t)n * nts + t], Tnt[(size_t)n * nts + nts - 1 - t]);
-      fold[(size_t)n * nth + t] = v;
-      fmax = std::max(fmax, std::max(std::fabs(v.x), std::fabs(v.y)));
-    }
+    for (int t = 0; t < nth; ++t)
+      tables[(size_t)n * nth + t] = cadd(Tnt[(size_t)n * nts + t], Tnt[(size_t)n * nts + nts - 1 - t]);
   Context::WTransforms& e = c.w_exact;
   e.nu = nw;
   e.nt = nts;
   e.bwd_host.assign(Ttn, Ttn + (size_t)nts * nw);
-  // frequencies with equal folded rows (each joins the first such one)
-  std::vector<int> group(nw, -1), first;
-  for (int n = 0; n < nw; ++n) {
-    for (size_t u = 0; u < first.size() && group[n] < 0; ++u) {
-      bool same = true;
-      for (int t = 0; same && t < nth; ++t) {
-        const cplx a = fold[(size_t)n * nth + t], b = fold[(size_t)first[u] * nth + t];
-        same = std::fabs(a.x - b.x) <= MIRROR_TOL * fmax && std::fabs(a.y - b.y) <= MIRROR_TOL * fmax;
-      }
-      if (same) group[n] = (int)u;
-    }
-    if (group[n] < 0) {
-      group[n] = (int)first.size();
-      first.push_back(n);
-    }
-  }
-  const int nu = (int)first.size();
-  std::vector<cplx> fwd((size_t)nu * nth, cmk(0.0, 0.0)), full((size_t)nts * nu, cmk(0.0, 0.0)), half((size_t)nth * nu);
-  std::vector<int> members(nu, 0);
-  for (int n = 0; n < nw; ++n) {
-    ++members[group[n]];
-    for (int t = 0; t < nth; ++t) {
-      cplx& f = fwd[(size_t)group[n] * nth + t];
-      f = cadd(f, fold[(size_t)n * nth + t]);
-    }
-    for (int t = 0; t < nts; ++t) {
-      cplx& f = full[(size_t)t * nu + group[n]];
-      f = cadd(f, Ttn[(size_t)t * nw + n]);
-    }
-  }
-  for (int u = 0; u < nu; ++u)
-    for (int t = 0; t < nth; ++t) fwd[(size_t)u * nth + t] = cscale(fwd[(size_t)u * nth + t], 1.0 / members[u]);
-  double asym = 0.0;
-  bool finite = true;
-  for (int t = 0; t < nth; ++t)
-    for (int u = 0; u < nu; ++u) {
-      const cplx a = full[(size_t)t * nu + u], b = full[(size_t)(nts - 1 - t) * nu + u];
-      bmax = std::max(bmax, std::max(std::max(std::fabs(a.x), std::fabs(a.y)), std::max(std::fabs(b.x), std::fabs(b.y))));
-      asym = std::max(asym, std::max(std::fabs(a.x - b.x), std::fabs(a.y - b.y)));
-      finite = finite && std::isfinite(a.x + a.y + b.x + b.y);
-      half[(size_t)t * nu + u] = cscale(cadd(a, b), 0.5);
-    }
+  const MirrorTransforms mt = mirror_transforms(reinterpret_cast<const host_cplx*>(tables.data()),
+                                                reinterpret_cast<const host_cplx*>(Ttn), nts, nw);
   Context::WTransforms& m = c.w_mirror;
-  m.nu = finite && asym <= MIRROR_TOL * bmax ? nu : 0;
+  m.nu = mt.ok ? mt.nu : 0;
   if (m.nu > 0) {
     m.nt = nth;
-    m.bwd_host = full;
-    fold.insert(fold.end(), fwd.begin(), fwd.end());
-    fold.insert(fold.end(), half.begin(), half.end());
+    auto dev = [](const std::vector<host_cplx>& v) { return reinterpret_cast<const cplx*>(v.data()); };
+    m.bwd_host.assign(dev(mt.full), dev(mt.full) + mt.full.size());
+    tables.insert(tables.end(), dev(mt.fwd), dev(mt.fwd) + mt.fwd.size());
+    tables.insert(tables.end(), dev(mt.half), dev(mt.half) + mt.half.size());
     std::vector<int64_t> tab((size_t)nts * ns);
     for (int t = 0; t < nts; ++t)
       for (int s = 0; s < ns; ++s)
@@ -258,12 +216,12 @@ void build_w_transforms(Context& c, const cplx* Tnt, const cplx* Ttn) {
     c.tab_x_mirror.upload(tab.data(), tab.size(), c.stream);
     GB_CUDA(cudaStreamSynchronize(c.stream));
   }
-  c.w_tables.upload(fold.data(), fold.size(), c.stream);
+  c.w_tables.upload(tables.data(), tables.size(), c.stream);
   GB_CUDA(cudaStreamSynchronize(c.stream));
   e.fwd = c.w_tables.get();
   e.bwd = c.Ttn_b.get();
   m.fwd = e.fwd + (size_t)nw * nth;
-  m.bwd = m.fwd + fwd.size();
+  m.bwd = m.fwd + (size_t)mt.nu * nth;
 }
 
 // Choose the k-block size so that the intermediates (and, without a caller's budget, the slice planes of the largest
