@@ -620,9 +620,10 @@ def main_batch(args):
         ctxs.append(c)
     b = batch.SystemBatch(ctxs)
     widths = b.apply_tiles()
-    # budgets cover the k-block intermediates; their INT8 planes take about 2S/16 of that again
+    # budgets hold the k-block intermediates and their INT8 planes (at five slices 5 bytes of planes for 6 of
+    # intermediates); W and the Dyson-sized buffers come on top
     free_b, _ = torch.cuda.mem_get_info(0)
-    b.share_memory(0.4 * free_b)
+    b.share_memory(0.55 * free_b)
     G = [torch.from_numpy(s.G).cuda() for s in systems]
     Sig = [torch.empty_like(x) for x in G]
     gp, sp = [x.data_ptr() for x in G], [x.data_ptr() for x in Sig]

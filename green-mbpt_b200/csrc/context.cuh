@@ -78,8 +78,8 @@ struct Context {
   int slices = 4;
   // slices of the P0 contractions (a)-(c) and the Sigma contractions (d)-(f); 0 takes `slices`
   int contraction_slices[6] = {0, 0, 0, 0, 0, 0};
-  // bytes the blocked intermediates of one call may take (GW: the two k-block buffers; HF: the
-  // exchange intermediates); 0 takes a default share of the free device memory
+  // bytes the blocked intermediates of one call may take (GW: the two k-block buffers and, in split precision, the
+  // slice planes; HF: the exchange intermediates); 0 takes a default share of the free device memory
   double mem_budget = 0.0;
   double budget_or(double cap, double free_share) const {
     if (mem_budget > 0.0) return mem_budget;

@@ -224,16 +224,6 @@ void build_w_transforms(Context& c, const cplx* Tnt, const cplx* Ttn) {
   m.bwd = m.fwd + (size_t)mt.nu * nth;
 }
 
-// Choose the k-block size so that the intermediates (and, without a caller's budget, the slice planes of the largest
-// contraction) fit the budget.
-static int choose_kblock(const Context& c, int64_t elems_per_k, int64_t plane_bytes_per_k) {
-  // leave headroom; at most 24 GB for the GW intermediates (40 GB with their planes) unless the caller set a budget
-  const double budget = c.budget_or(plane_bytes_per_k > 0 ? 40e9 : 24e9, 0.6);
-  double per_k = (double)elems_per_k * sizeof(cplx) + (c.mem_budget > 0.0 ? 0.0 : (double)plane_bytes_per_k);
-  int kb = (int)std::max(1.0, std::floor(budget / per_k));
-  return std::min(kb, c.d.nk);
-}
-
 cplx extrapolate_q0(const cplx* eps_n, const std::vector<double>& q_abs, int fit_order, double q_max) {
   // first occurrence of every distinct |q| in (0, q_max] (filter_q_abs), quadratic least squares
   // by the normal equations solved with full pivoting (polyfit); rank-deficient systems take 0
@@ -405,16 +395,35 @@ struct GwRun {
     by_z = nh * ns > 1;
     acc = nh == 2 ? (cplx*)c.scratch.get(SL_SIG_FOLD, (size_t)nts * ns * nk * nao2 * sizeof(cplx)) : Sigma;
     GB_CUDA(cudaMemsetAsync(acc, 0, (size_t)nts * ns * nk * nao2 * sizeof(cplx), st));
-    const int64_t x1_k = (int64_t)nts * ns * pe;
-    const int64_t x2_k = by_z ? std::max((int64_t)nth * ns, (int64_t)ntz) * pe : x1_k;
-    // planes of (f): 2 bytes a slice and element of the right operand, 4 of the left one
-    const int64_t planes_k = !split ? 0 : 2 * slices_of(5) * (by_z ? x1_k + 2 * (int64_t)ntz * pe : x1_k);
-    kb = choose_kblock(c, x1_k + x2_k, planes_k);
-    kb = std::min<int64_t>(kb, std::max<int64_t>(1, 65535 / ((int64_t)nts * ns)));  // batches of one launch
     P0 = (cplx*)c.scratch.get(SL_P0, (size_t)nts * NQ * NQ * sizeof(cplx));
     Pw = (cplx*)c.scratch.get(SL_PW, (size_t)nw_b * NQ * NQ * sizeof(cplx));
     Pinv = (cplx*)c.scratch.get(SL_PINV, (size_t)nw_b * NQ * NQ * sizeof(cplx));
     aug = (cplx*)c.scratch.get(SL_AUG, (size_t)nw_b * NQ * 2 * NQ * sizeof(cplx));
+    // the largest k-block whose two intermediates and, in split precision, slice planes fit the budget: the caller's, or
+    // 24 GB (40 GB with planes) and 0.6 of what is free
+    const int64_t x1_k = (int64_t)nts * ns * pe;
+    const int64_t x2_k = by_z ? std::max((int64_t)nth * ns, (int64_t)ntz) * pe : x1_k;
+    SplitBuffers planes;
+    auto need = [&](int k) {  // bytes of blocks of k k-points; sets `planes`
+      kb = k;
+      planes = SplitBuffers();
+      if (split) {
+        ZGemm g3[3];
+        p0_gemms(0, 0, g3);
+        for (int i = 0; i < 3; ++i) planes.cover(g3[i], slices_of(i));
+        sigma_gemms(0, 0, g3);
+        for (int i = 0; i < 3; ++i) planes.cover(g3[i], slices_of(3 + i));
+      }
+      return (double)k * (double)(x1_k + x2_k) * sizeof(cplx) + (double)planes.bytes();
+    };
+    const double budget = c.budget_or(split ? 40e9 : 24e9, 0.6);
+    int lo = 1, hi = (int)std::min<int64_t>(nk, std::max<int64_t>(1, 65535 / ((int64_t)nts * ns)));  // (batches of one launch)
+    while (lo < hi) {
+      const int mid = (lo + hi + 1) / 2;
+      if (need(mid) <= budget) lo = mid;
+      else hi = mid - 1;
+    }
+    need(lo);
     X1 = (cplx*)c.scratch.get(SL_Y1, (size_t)kb * x1_k * sizeof(cplx));
     X2 = (cplx*)c.scratch.get(SL_Y2, (size_t)kb * x2_k * sizeof(cplx));
     if (c.q0_on) {

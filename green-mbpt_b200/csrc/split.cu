@@ -1328,6 +1328,10 @@ int tile_width(const Context& c, int S, int64_t M, bool overlap) {
   return best;
 }
 
+// bytes of a plane's row for Kc complex K positions: whole 32-byte K steps of the MMA; a last half block is filled with
+// zeros by the TMA load
+int64_t row_bytes(int64_t Kc) { return std::max<int64_t>(KBLK, rup(2 * Kc, 32)); }
+
 struct Prepared {
   GemmParams p{};
   CUtensorMap mR{}, mC{};
@@ -1349,12 +1353,13 @@ Prepared prepare_chunk(SplitEngine& se, const ZGemm& g0, int S, int BN, int64_t 
     se.err.alloc(1);
     GB_CUDA(cudaMemsetAsync(se.err.p, 0, sizeof(int), st));
   }
-  // whole 32-byte K steps of the MMA; a last half block is filled with zeros by the TMA load
-  const int64_t kpad = std::max<int64_t>(KBLK, rup(2 * Kc, 32));
-  se.planesA.alloc((size_t)(nrbA * S * rowsA * kpad));
-  se.planesB.alloc((size_t)(nrbB * S * rowsB * kpad));
-  se.expA.alloc((size_t)(nrbA * g0.M));
-  se.expB.alloc((size_t)(nrbB * g0.N));
+  const int64_t kpad = row_bytes(Kc);
+  SplitBuffers buf;
+  buf.cover(g0, S);
+  se.planesA.alloc(buf.planesA);
+  se.planesB.alloc(buf.planesB);
+  se.expA.alloc(buf.expA);
+  se.expB.alloc(buf.expB);
   auto slice = [&](const ZOperand& o, const IdxMap& rmap, const IdxMap& kmap, const int* dep, int64_t R, int64_t nrb,
                    int embed, int8_t* out, int32_t* expo) {
     SliceJob j{};
@@ -1462,6 +1467,17 @@ unsigned persistent_grid(const Context& c, int64_t ntiles) {
 }
 
 }  // namespace
+
+void SplitBuffers::cover(const ZGemm& g, int S) {
+  int depA[3], depB[3];
+  deps_of(g.A, depA);
+  deps_of(g.B, depB);
+  const int64_t nrbA = nrb_of(depA, g), nrbB = nrb_of(depB, g), kpad = row_bytes(std::min(kmax_for(S), g.K));
+  planesA = std::max(planesA, (size_t)(nrbA * S * 2 * g.M * kpad));
+  planesB = std::max(planesB, (size_t)(nrbB * S * g.N * kpad));
+  expA = std::max(expA, (size_t)(nrbA * g.M));
+  expB = std::max(expB, (size_t)(nrbB * g.N));
+}
 
 void split_gemm(Context& c, SplitEngine& se, const ZGemm& g0, cudaStream_t st, int slices) {
   if (g0.M <= 0 || g0.N <= 0) return;

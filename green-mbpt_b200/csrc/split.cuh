@@ -20,6 +20,14 @@ void split_gemm(Context& c, SplitEngine& se, const ZGemm& g, cudaStream_t st, in
 // persistent tensor-core launch per K chunk walks the tiles of all of them.
 void split_gemm_group(const std::vector<Context*>& cs, const std::vector<ZGemm>& gs, cudaStream_t st, int slices);
 void split_release(Context& c);
+
+// What contractions take of the engine's buffers: slice planes (bytes) and exponents (counts) of the left and the right
+// operand, each the largest of the contractions covered.  Only the shape of a descriptor is read.
+struct SplitBuffers {
+  size_t planesA = 0, planesB = 0, expA = 0, expB = 0;
+  void cover(const ZGemm& g, int slices);
+  size_t bytes() const { return planesA + planesB + (expA + expB) * sizeof(int32_t); }
+};
 // Non-zero if a split kernel hit a bounded-wait timeout since the last check (flag is cleared).
 int split_check_error(Context& c, cudaStream_t st);
 

@@ -31,9 +31,10 @@ class SystemBatch:
         return len(self.contexts)
 
     def share_memory(self, total_bytes: float):
-        """Give every context a budget for its blocked intermediates out of `total_bytes`, in
-        proportion to the size of one k-point block of its self-energy intermediates
-        (nts * ns * NQ * nao^2 complex values), so that all contexts fit on one GPU together."""
+        """Give every context a budget for its blocked intermediates and their slice planes out of
+        `total_bytes`, in proportion to the size of one k-point block of its self-energy intermediates
+        (nts * ns * NQ * nao^2 complex values), so that all contexts fit on one GPU together: the
+        integrals and the buffers of fixed size come on top."""
         sizes = []
         for c in self.contexts:
             d = c.dims

@@ -152,8 +152,9 @@ int gb200_set_precision(gb200_context* ctx, int mode, int slices);
 int gb200_set_contraction_slices(gb200_context* ctx, const int* slices6);
 
 /* Bytes the blocked intermediates of one call may use (the k-block buffers of the GW self-energy
- * and its adjoint, the exchange intermediates of the Fock build); 0 (the default) takes a share of
- * the free device memory at the call.  For several contexts sharing one GPU.  The reference sizes
+ * and its adjoint, in split precision the slice planes of their contractions too, the exchange
+ * intermediates of the Fock build), but at least one k-point's worth; 0 (the default) takes a share
+ * of the free device memory at the call.  For several contexts sharing one GPU.  The reference sizes
  * its buffers per MPI rank instead (gw_cpu_kernel.cpp:74-134); no counterpart. */
 int gb200_set_memory_budget(gb200_context* ctx, double bytes);
 
