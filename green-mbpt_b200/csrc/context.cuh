@@ -48,6 +48,7 @@ struct Scratch {
     bufs[slot]->alloc(bytes);
     return bufs[slot]->p;
   }
+  size_t held(int slot) const { return (int)bufs.size() > slot && bufs[slot] ? bufs[slot]->n : 0; }
   void release() { bufs.clear(); }
 };
 
@@ -79,13 +80,14 @@ struct Context {
   // slices of the P0 contractions (a)-(c) and the Sigma contractions (d)-(f); 0 takes `slices`
   int contraction_slices[6] = {0, 0, 0, 0, 0, 0};
   // bytes the blocked intermediates of one call may take (GW: the two k-block buffers and, in split precision, the
-  // slice planes; HF: the exchange intermediates); 0 takes a default share of the free device memory
+  // slice planes; HF: the exchange intermediates); 0 takes a default share of the free device memory.  `held`: what the
+  // same buffers hold from an earlier call, which is as good as free; without it a later call would choose smaller blocks.
   double mem_budget = 0.0;
-  double budget_or(double cap, double free_share) const {
+  double budget_or(double cap, double free_share, size_t held) const {
     if (mem_budget > 0.0) return mem_budget;
     size_t free_b = 0, total_b = 0;
     GB_CUDA(cudaMemGetInfo(&free_b, &total_b));
-    return std::min(cap, free_share * (double)free_b);
+    return std::min(cap, free_share * ((double)free_b + (double)held));
   }
   int split_core = 0;             // 0: tcgen05 tensor cores, 1: CUDA-core validation core
   int tile_bn = 0;                // column tile of the split contractions (0: the widest that fits)

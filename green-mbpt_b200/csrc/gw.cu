@@ -416,7 +416,8 @@ struct GwRun {
       }
       return (double)k * (double)(x1_k + x2_k) * sizeof(cplx) + (double)planes.bytes();
     };
-    const double budget = c.budget_or(split ? 40e9 : 24e9, 0.6);
+    const size_t held = c.scratch.held(SL_Y1) + c.scratch.held(SL_Y2) + (split ? split_held(c) : 0);
+    const double budget = c.budget_or(split ? 40e9 : 24e9, 0.6, held);
     int lo = 1, hi = (int)std::min<int64_t>(nk, std::max<int64_t>(1, 65535 / ((int64_t)nts * ns)));  // (batches of one launch)
     while (lo < hi) {
       const int mid = (lo + hi + 1) / 2;

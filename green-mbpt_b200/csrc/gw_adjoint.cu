@@ -142,7 +142,8 @@ void gw_sigma_vjp(Context& c, const cplx* G, const cplx* Sb, cplx* Gb, cplx* Vb,
   cplx* P0hb = buf(SL_ADJ_P0HB, nth * nq2);
   // k-block: three intermediates of nts*ns*pe per k-point
   const int64_t blk = (int64_t)nts * ns * pe;
-  const double budget = c.budget_or(24e9, 0.6);
+  const double budget =
+      c.budget_or(24e9, 0.6, c.scratch.held(SL_Y1) + c.scratch.held(SL_Y2) + c.scratch.held(SL_ADJ_X3));
   int kb = (int)std::max(1.0, std::floor(budget / (3.0 * (double)blk * sizeof(cplx))));
   kb = std::min(kb, nk);
   cplx* X1 = buf(SL_Y1, kb * blk);

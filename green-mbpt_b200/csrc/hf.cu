@@ -187,7 +187,7 @@ static void hf_core(Context& c, const cplx* V, const cplx* dm, int nsp, int ndir
   // order by exchange_reduce_kernel, so the result is deterministic.
   if (!sub) {
     const int64_t per_k = (int64_t)nsp * nk * pe;
-    const double budget = c.budget_or(8e9, 0.5);
+    const double budget = c.budget_or(8e9, 0.5, c.scratch.held(SL_HF_Y));
     int kb = (int)std::max(1.0, std::floor(budget / ((double)per_k * sizeof(cplx))));
     kb = std::min(kb, nk);
     cplx* Y = (cplx*)c.scratch.get(SL_HF_Y, (size_t)kb * per_k * sizeof(cplx));

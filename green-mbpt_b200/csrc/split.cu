@@ -1479,6 +1479,12 @@ void SplitBuffers::cover(const ZGemm& g, int S) {
   expB = std::max(expB, (size_t)(nrbB * g.N));
 }
 
+size_t split_held(const Context& c) {
+  if (!c.split) return 0;
+  const SplitEngine& e = *c.split;
+  return e.planesA.n + e.planesB.n + (e.expA.n + e.expB.n) * sizeof(int32_t);
+}
+
 void split_gemm(Context& c, SplitEngine& se, const ZGemm& g0, cudaStream_t st, int slices) {
   if (g0.M <= 0 || g0.N <= 0) return;
   validate(g0);

@@ -1,5 +1,6 @@
 """Device memory of the blocked self-energy: what a call allocates beyond its fixed buffers stays within the budget that
-the caller set, digit planes included."""
+the caller set, digit planes included, and without a budget the buffers of one call do not make the next one choose
+smaller blocks."""
 import gc
 
 import numpy as np
@@ -40,3 +41,27 @@ def test_blocks_and_planes_stay_within_the_budget(gpu, ns, nao, naux, slices):
         # (`single` holds a block too: room for the granules of a few dozen allocations)
         assert got - single <= budget
         assert np.abs(out - ref).max() <= 1e-8 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("slices", [0, 5])
+def test_a_second_call_takes_the_same_blocks(gpu, slices):
+    """With memory for about half of the k-points: the same launches and the same bits, call after call."""
+    import torch
+    s = synth.make_system(mesh=(4, 2, 2), nao=24, naux=140, ns=1, beta=20.0, nts=80, eps_range=2.0, seed=1)
+    per_k = 16.0 * 80 * 140 * 24 * 24 * (2.75 if slices else 2.0)
+    with solvers.make_context(s, precision=lib.PREC_SPLIT if slices else lib.PREC_FP64, slices=slices or 4) as c:
+        c.set_memory_budget(1.0)
+        c.gw_sigma(s.G)  # the kernels and the buffers of fixed size
+        c.set_memory_budget(0.0)
+        ballast = torch.empty(int(_free() - 8 * per_k / 0.6), dtype=torch.uint8, device="cuda")
+        try:
+            out, launches = [], []
+            for _ in range(3):
+                before = c.stats_read()[0]
+                out.append(c.gw_sigma(s.G))
+                launches.append(c.stats_read()[0] - before)
+        finally:
+            del ballast
+            torch.cuda.empty_cache()
+    assert launches[0] == launches[1] == launches[2]
+    assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
