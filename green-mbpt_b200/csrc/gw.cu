@@ -427,6 +427,8 @@ struct GwRun {
     need(lo);
     X1 = (cplx*)c.scratch.get(SL_Y1, (size_t)kb * x1_k * sizeof(cplx));
     X2 = (cplx*)c.scratch.get(SL_Y2, (size_t)kb * x2_k * sizeof(cplx));
+    // (at once: the next context of a batched call must not count the planes' memory as free)
+    if (split) split_reserve(c, planes);
     if (c.q0_on) {
       require(c.q_begin <= 0 && (c.q_end < 0 || c.q_end >= nk), GB200_ERR_INVALID,
               "q0 correction: needs all q-points in one context (it extrapolates over q)");

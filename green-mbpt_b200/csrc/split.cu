@@ -1479,6 +1479,14 @@ void SplitBuffers::cover(const ZGemm& g, int S) {
   expB = std::max(expB, (size_t)(nrbB * g.N));
 }
 
+void split_reserve(Context& c, const SplitBuffers& b) {
+  SplitEngine& e = *split_engine(c);
+  e.planesA.alloc(b.planesA);
+  e.planesB.alloc(b.planesB);
+  e.expA.alloc(b.expA);
+  e.expB.alloc(b.expB);
+}
+
 size_t split_held(const Context& c) {
   if (!c.split) return 0;
   const SplitEngine& e = *c.split;

@@ -28,6 +28,8 @@ struct SplitBuffers {
   void cover(const ZGemm& g, int slices);
   size_t bytes() const { return planesA + planesB + (expA + expB) * sizeof(int32_t); }
 };
+// allocate them in the context's engine
+void split_reserve(Context& c, const SplitBuffers& b);
 // bytes that a context's engine holds in these buffers
 size_t split_held(const Context& c);
 // Non-zero if a split kernel hit a bounded-wait timeout since the last check (flag is cleared).

@@ -6,7 +6,7 @@ import gc
 import numpy as np
 import pytest
 
-from gb200 import lib, solvers, synth
+from gb200 import batch, lib, solvers, synth
 
 pytestmark = pytest.mark.gpu
 
@@ -65,3 +65,32 @@ def test_a_second_call_takes_the_same_blocks(gpu, slices):
             torch.cuda.empty_cache()
     assert launches[0] == launches[1] == launches[2]
     assert np.array_equal(out[0], out[1]) and np.array_equal(out[0], out[2])
+
+
+def test_contexts_of_one_batched_call_share_what_is_free(gpu):
+    """Four systems whose blocks would each take most of the free memory, without budgets: together they fit."""
+    import torch
+    systems = [synth.make_system(mesh=(4, 2, 2), nao=24, naux=140, ns=1, beta=20.0, nts=80, eps_range=2.0, seed=i) for i in range(4)]
+    per_k = 16.0 * 80 * 140 * 24 * 24 * 2.75
+    ctxs = [solvers.make_context(s, precision=lib.PREC_SPLIT, slices=5) for s in systems]
+    try:
+        b = batch.SystemBatch(ctxs)
+        G = [torch.from_numpy(s.G).cuda() for s in systems]
+        Sig = [torch.empty_like(g) for g in G]
+        gp, sp = [x.data_ptr() for x in G], [x.data_ptr() for x in Sig]
+        with solvers.make_context(systems[0], precision=lib.PREC_SPLIT, slices=5) as c:
+            c.set_memory_budget(1.0)
+            before = _free()
+            ref = c.gw_sigma(systems[0].G)
+            single = before - _free()  # one context's fixed buffers and a block of one k-point
+        ballast = torch.empty(int(_free() - 12 * per_k - 4 * single), dtype=torch.uint8, device="cuda")
+        try:
+            b.run_gw_grouped(gp, sp)
+            torch.cuda.synchronize()
+        finally:
+            del ballast
+            torch.cuda.empty_cache()
+        assert np.abs(Sig[0].cpu().numpy() - ref).max() <= 1e-8 * np.abs(ref).max()
+    finally:
+        for c in ctxs:
+            c.close()
