@@ -191,14 +191,13 @@ void energy(Context& c, const cplx* G, const cplx* Sigma1, const cplx* Sigma_tau
 
 // linear algebra helpers (linalg.cu)
 void hermitize_batched(cplx* X, int64_t nmat, int n, double scale, cudaStream_t st);
-void invert_small_batched(const cplx* A, cplx* Ainv, int64_t nmat, int n, cudaStream_t st);
 // G[w][sk] = (z_w S[sk] - X[w][sk])^-1 with z_w = mu + i wn[w], and tr[w][sk] = Tr(G[w][sk] S[sk])
 void invert_dyson_batched(const cplx* X, const cplx* S, const double* wn, double mu, cplx* G, int64_t nw, int64_t nsk,
                           int n, cudaStream_t st);
 void trace_dyson_batched(const cplx* X, const cplx* S, const double* wn, double mu, cplx* tr, int64_t nw, int64_t nsk,
                          int n, cudaStream_t st);
 // Inverse of the Hermitian matrix that the lower triangle and real diagonal of A (or I - A) define; `aug` holds
-// nmat * 2 n^2 elements, `bad` nmat flags.  The result is Hermitian.
+// nmat * 2 n^2 elements, `bad` nmat flags.  The result is Hermitian up to rounding (exactly so from the block inverse).
 void invert_large_batched(const cplx* A, cplx* Ainv, cplx* aug, int* bad, int64_t nmat, int n, bool identity_minus,
                           cudaStream_t st);
 void scale_inplace(cplx* X, int64_t count, double s, cudaStream_t st);

@@ -119,7 +119,8 @@ __device__ __forceinline__ bool gj_invert(cplx (&m)[RI][CJ], int n, GjShared& sh
       int p = k;
       if constexpr (PIVOT) {
         __syncthreads();
-        // the high words of non-negative doubles order like the numbers; ties go to the smaller row
+        // the high words of non-negative doubles order like the numbers; ties (within 2^-20) go to the lowest lane, and
+        // to the smaller row of a lane's two
         int best = -1, row = 0;
 #pragma unroll
         for (int h = 0; h < (RI * TI > 32 ? 2 : 1); ++h) {
@@ -201,7 +202,6 @@ __device__ __forceinline__ bool gj_invert(cplx (&m)[RI][CJ], int n, GjShared& sh
 
 // What a CTA inverts and what becomes of the result.
 enum GjMode {
-  GJ_GENERAL,  // A -> Ainv, partial pivoting
   GJ_HERM,     // the Hermitian matrix of the lower triangle and real diagonal of A or I - A -> Ainv, with pivoting
   GJ_LEAF,     // a positive definite diagonal block in place; bad[matrix] = 1 if it is not
   GJ_DYSON,    // z S - X -> Ainv, z = mu + i w of the matrix's frequency
@@ -306,7 +306,7 @@ void launch_gj_one(const GjJob& j, cudaStream_t st) {
 // interaction one per frequency.
 template <int MODE>
 void launch_gj(const GjJob& j, int64_t nmat, cudaStream_t st) {
-  constexpr bool many = MODE == GJ_GENERAL || MODE == GJ_DYSON || MODE == GJ_TRACE;
+  constexpr bool many = MODE == GJ_DYSON || MODE == GJ_TRACE;
   for (int64_t off = 0; off < nmat; off += 2147483647LL) {
     GjJob q = j;
     q.nmat = std::min<int64_t>(nmat - off, 2147483647LL);
@@ -369,9 +369,8 @@ __global__ void herm_join_kernel(cplx* B, int64_t nmat, int n, int off, int size
 constexpr int LARGE_NT = 1024;
 
 __global__ void __launch_bounds__(LARGE_NT) invert_large_kernel(const cplx* A, cplx* Ainv, cplx* augbase, int n,
-                                                                 bool herm_from_lower, bool identity_minus,
-                                                                 const int* bad) {
-  if (bad && !bad[blockIdx.x]) return;
+                                                                 bool identity_minus, const int* bad) {
+  if (!bad[blockIdx.x]) return;
   extern __shared__ double2 smem_c[];
   cplx* prow = smem_c;           // 2n (pivot row)
   cplx* fac = prow + 2 * n;      // n
@@ -383,21 +382,16 @@ __global__ void __launch_bounds__(LARGE_NT) invert_large_kernel(const cplx* A, c
   const cplx* Am = A + m * (int64_t)n * n;
   for (int64_t e = threadIdx.x; e < (int64_t)n * n; e += LARGE_NT) {
     int i = (int)(e / n), c = (int)(e % n);
-    // B = identity_minus ? I - A : A ; the inverted matrix is B itself or, with
-    // herm_from_lower, the Hermitian matrix of B's strict lower triangle and
-    // real diagonal (what Eigen's LDLT reads, gw_cpu_kernel.cpp:245-249)
+    // B = identity_minus ? I - A : A ; the inverted matrix is the Hermitian one of B's strict lower triangle and real
+    // diagonal (what Eigen's LDLT reads, gw_cpu_kernel.cpp:245-249)
     auto Bel = [&](int x, int y) -> cplx {
       cplx a = Am[(int64_t)x * n + y];
       return identity_minus ? cmk((x == y ? 1.0 : 0.0) - a.x, -a.y) : a;
     };
     cplx v;
-    if (herm_from_lower) {
-      if (i > c) v = Bel(i, c);
-      else if (i < c) v = cconj(Bel(c, i));
-      else v = cmk(Bel(i, i).x, 0.0);
-    } else {
-      v = Bel(i, c);
-    }
+    if (i > c) v = Bel(i, c);
+    else if (i < c) v = cconj(Bel(c, i));
+    else v = cmk(Bel(i, i).x, 0.0);
     aug[(int64_t)i * ld + c] = v;
     aug[(int64_t)i * ld + n + c] = (i == c) ? cmk(1.0, 0.0) : cmk(0.0, 0.0);
   }
@@ -465,9 +459,8 @@ __device__ __forceinline__ void block_argmax(double v, int idx, double* sval, in
 }
 
 __global__ void __launch_bounds__(BLK_NT) invert_blocked_kernel(const cplx* A, cplx* Ainv, cplx* augbase, int n,
-                                                                bool herm_from_lower, bool identity_minus,
-                                                                const int* bad) {
-  if (bad && !bad[blockIdx.x]) return;
+                                                                bool identity_minus, const int* bad) {
+  if (!bad[blockIdx.x]) return;
   extern __shared__ double2 smem_c[];
   cplx* pan = smem_c;                        // [n][BLK_NB]: panel copy, then the original panel rows
   cplx* dinv = pan + (size_t)n * BLK_NB;     // [BLK_NB][2*BLK_NB]: D | I -> I | D^-1
@@ -486,13 +479,9 @@ __global__ void __launch_bounds__(BLK_NT) invert_blocked_kernel(const cplx* A, c
       return identity_minus ? cmk((x == y ? 1.0 : 0.0) - a.x, -a.y) : a;
     };
     cplx v;
-    if (herm_from_lower) {
-      if (i > c) v = Bel(i, c);
-      else if (i < c) v = cconj(Bel(c, i));
-      else v = cmk(Bel(i, i).x, 0.0);
-    } else {
-      v = Bel(i, c);
-    }
+    if (i > c) v = Bel(i, c);
+    else if (i < c) v = cconj(Bel(c, i));
+    else v = cmk(Bel(i, i).x, 0.0);
     aug[(int64_t)i * ld + c] = v;
     aug[(int64_t)i * ld + n + c] = (i == c) ? cmk(1.0, 0.0) : cmk(0.0, 0.0);
   }
@@ -653,14 +642,6 @@ void scale_inplace(cplx* X, int64_t count, double s, cudaStream_t st) {
   GB_CHECK_LAUNCH();
 }
 
-void invert_small_batched(const cplx* A, cplx* Ainv, int64_t nmat, int n, cudaStream_t st) {
-  require(n <= 64, GB200_ERR_INVALID, "invert_small_batched: n > 64");
-  if (nmat <= 0) return;
-  GjJob j;
-  j.A = A; j.out = Ainv; j.stride = (int64_t)n * n; j.ld = n; j.n = n;
-  launch_gj<GJ_GENERAL>(j, nmat, st);
-}
-
 void invert_dyson_batched(const cplx* X, const cplx* S, const double* wn, double mu, cplx* G, int64_t nw, int64_t nsk,
                           int n, cudaStream_t st) {
   require(n <= 64, GB200_ERR_INVALID, "invert_dyson_batched: n > 64");
@@ -752,10 +733,10 @@ void invert_large_batched(const cplx* A, cplx* Ainv, cplx* aug, int* bad, int64_
   GB_CUDA(cudaFuncSetAttribute(invert_blocked_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, 220 * 1024));
   const size_t bsmem = blocked_smem_bytes(n);
   if (bsmem <= 220 * 1024) {
-    invert_blocked_kernel<<<(unsigned)nmat, BLK_NT, bsmem, st>>>(A, Ainv, aug, n, true, identity_minus, bad);
+    invert_blocked_kernel<<<(unsigned)nmat, BLK_NT, bsmem, st>>>(A, Ainv, aug, n, identity_minus, bad);
   } else {
     const size_t smem = (size_t)(3 * n) * sizeof(cplx);
-    invert_large_kernel<<<(unsigned)nmat, LARGE_NT, smem, st>>>(A, Ainv, aug, n, true, identity_minus, bad);
+    invert_large_kernel<<<(unsigned)nmat, LARGE_NT, smem, st>>>(A, Ainv, aug, n, identity_minus, bad);
   }
   GB_CHECK_LAUNCH();
 }
