@@ -1292,7 +1292,6 @@ void run_slicer(SliceJob& j, int64_t nrb, cudaStream_t st) {
   GB_CHECK_LAUNCH();
   dim3 g2((unsigned)((j.rpad + TR - 1) / TR), (unsigned)((j.kpad / 2 + TK - 1) / TK), (unsigned)nrb);
   launch_write(j, g2, st);
-  GB_CHECK_LAUNCH();
   fix_empty_expo_kernel<<<blocks_for(ne), 256, 0, st>>>(j.expo, ne);
   GB_CHECK_LAUNCH();
 }
