@@ -595,7 +595,7 @@ def main_newton(args):
 def main_batch(args):
     """--batch N: N independent systems of uneven sizes (gb200.batch.uneven_systems: nk from {8, 27, 64},
     nao ~ U{8..48}, naux ~ U{4 nao..6 nao}, ntau = 80, beta = 100), integrals generated on the device,
-    one context per system with memory budgets in proportion to their intermediates, tile widths from
+    one context per system with memory budgets in proportion to their intermediates, tile width limits from
     the autotuner's table (gb200/tile_table.json), split precision.  The timed call is
     gb200_gw_sigma_batch_device: the systems' q-points in step, every contraction stage one grouped
     persistent tensor-core launch over the tiles of all systems (CUDA events).  The same batch issued
@@ -662,7 +662,7 @@ def main_batch(args):
                                 f"mean of {args.steps} after {args.warmup} warm-up",
                       "wall_seconds_per_batch": grouped_wall,
                       "thread_pool_seconds_per_batch": pool_wall,
-                      "tile_widths": "gb200/tile_table.json (0: widest)",
+                      "tile_widths": "upper limits from gb200/tile_table.json (0: none)",
                       "systems": rows}), flush=True)
     b.close()
 
@@ -730,7 +730,7 @@ def parse(argv=None):
     ap.add_argument("--profile-fp64", dest="profile_fp64", action="store_true",
                     help="profiling case in FP64 instead of split precision")
     ap.add_argument("--tile-width", dest="tile_width", type=int, default=0,
-                    help="profiling case: column tile of the tensor-core contractions (0: the default)")
+                    help="profiling case: upper limit of the tensor-core contractions' column tile (0: none)")
     ap.add_argument("--newton", type=int, default=0,
                     help="differentiable-step case (--config c4): adjoint timings, then N plain and N "
                          "Newton-Krylov self-consistency steps from the same start")

@@ -340,7 +340,7 @@ int gb200_gw_sigma_batch_device(gb200_context* const* ctxs, int n, const double*
 
 int gb200_set_tile_width(gb200_context* ctx, int bn) {
   return guarded(ctx, [&](Context& c) {
-    require(bn >= 0 && bn <= 256, GB200_ERR_INVALID, "set_tile_width: 0 (widest) or a width up to 256");
+    require(bn >= 0 && bn <= 256, GB200_ERR_INVALID, "set_tile_width: 0 (no limit) or a width up to 256");
     c.tile_bn = bn;
   });
 }

@@ -90,7 +90,7 @@ struct Context {
     return std::min(cap, free_share * ((double)free_b + (double)held));
   }
   int split_core = 0;             // 0: tcgen05 tensor cores, 1: CUDA-core validation core
-  int tile_bn = 0;                // column tile of the split contractions (0: the widest that fits)
+  int tile_bn = 0;                // upper limit of the split contractions' column tile (0: none)
   SplitEngine* split = nullptr;
 
   bool have_kq = false, have_grid = false, have_V = false, have_Vhf = false, have_H = false;

@@ -3,11 +3,10 @@
 Each system keeps its own context: its integrals, grid, maps and scratch buffers, and its own
 CUDA stream.  `run_gw_grouped` evaluates all of them in one library call whose contraction stages
 are grouped persistent launches over the tiles of every system (gb200_gw_sigma_batch_device), with
-tile widths from the autotuner's table (`apply_tiles`).  `run_gw` instead issues the self-energy of
-every system from a pool of host threads.  The
-library calls release the interpreter lock, so the systems' kernels are queued on different
-streams and overlap on the device wherever one system does not fill it: the slicing and FP64
-kernels of one system run beside the contraction kernel of another.  Results are identical to
+limits of the tile width from the autotuner's table (`apply_tiles`).  `run_gw` instead issues the
+self-energy of every system from a pool of host threads.  The library calls release the
+interpreter lock, so the systems' kernels are queued on different streams and
+overlap on the device wherever one system does not fill it: the slicing and FP64 kernels of one system run beside the contraction kernel of another.  Results are identical to
 running the systems one by one: every context computes exactly what it would alone.
 """
 from __future__ import annotations
@@ -69,7 +68,7 @@ class SystemBatch:
         lib.gw_sigma_batch_device(self.contexts, G_ptrs, Sigma_ptrs, stream)
 
     def apply_tiles(self, table=None):
-        """Tile width of every context from the autotuner's table (gb200.tune.choose_tile)."""
+        """Limit of the tile width of every context from the autotuner's table (gb200.tune.choose_tile)."""
         from . import tune
         widths = []
         for c in self.contexts:

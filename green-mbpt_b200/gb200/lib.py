@@ -306,7 +306,7 @@ class Context:
                                                        ctypes.c_void_p(stream)))
 
     def set_tile_width(self, bn: int = 0):
-        """Column tile of the split-precision contractions (0: the widest that fits)."""
+        """Upper limit of the split-precision contractions' column tile (0: none)."""
         self._check(self._L.gb200_set_tile_width(self._h, int(bn)))
 
     def set_integrals_pairs(self, V_pairs, pair_ids, stream: int = 0):

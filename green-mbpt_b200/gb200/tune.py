@@ -1,12 +1,15 @@
 """Tile-width autotuner for the split-precision contractions, per (nao, naux).
 
-The column tile of the tensor-core contraction kernel (gb200_set_tile_width) trades the width of
-one MMA against tile-count rounding of each contraction's N (N = naux nao, naux, nk nao^2 or
-ntau nao) and the per-tile epilogue work.  `measure` times the whole self-energy of a synthetic
-system of the given (nao, naux) with every candidate width (CUDA events, after warm-up);
-`tune` does so over a grid of shapes and `tile_table.json` next to this file holds the result of a
-run on a B200 (python -m gb200.tune --out ...).  `choose_tile` reads the table: the entry of the
-nearest measured shape (relative distance in nao and naux), 0 (the widest tile) without one.
+The columns of the tensor-core contraction kernel's tile are the real embedding of a contraction's
+smaller operand (2 M columns, M = ntau nao, nao, naux or nao^2).  The library chooses their number
+per contraction by a cost rule, between half of the widest tile that the slices leave room for and
+that tile; gb200_set_tile_width puts an upper limit on it for all six contractions, which pays
+where a system is better off with more and narrower tiles than the rule expects.  `measure` times
+the whole self-energy of a synthetic system of the given (nao, naux) with every candidate limit
+(CUDA events, in turn, after warm-up), 0 being the rule alone; `tune` does so over a grid of shapes and
+`tile_table.json` next to this file holds the result of a run on a B200 (python -m gb200.tune
+--out ...).  `choose_tile` reads the table: the entry of the nearest measured shape (relative
+distance in nao and naux), 0 without one.
 """
 from __future__ import annotations
 
@@ -15,7 +18,7 @@ import json
 import math
 import os
 
-CANDIDATES = (32, 48, 64, 80, 96)
+CANDIDATES = (0, 32, 48, 64, 80)  # (96 is the widest tile of five slices, so no limit)
 TABLE = os.path.join(os.path.dirname(os.path.abspath(__file__)), "tile_table.json")
 
 
@@ -27,7 +30,7 @@ def load_table(path: str = TABLE) -> dict:
 
 
 def choose_tile(nao: int, naux: int, table: dict | None = None) -> int:
-    """Tile width for a system of (nao, naux) from the measured table (0: widest)."""
+    """Limit of the tile width for a system of (nao, naux) from the measured table (0: none)."""
     table = load_table() if table is None else table
     best, dist = 0, math.inf
     for key, entry in table.items():
@@ -38,9 +41,9 @@ def choose_tile(nao: int, naux: int, table: dict | None = None) -> int:
     return best
 
 
-def measure(nao: int, naux: int, slices: int = 5, nts: int = 80, mesh=(2, 2, 2), reps: int = 3,
+def measure(nao: int, naux: int, slices: int = 5, nts: int = 80, mesh=(2, 2, 2), reps: int = 9,
             candidates=CANDIDATES, seed: int = 0, device: int = 0) -> dict:
-    """Milliseconds of one split-precision self-energy of a synthetic system per tile width."""
+    """Milliseconds (the fastest of `reps`) of one split-precision self-energy of a synthetic system per limit of the tile width."""
     import torch
 
     from . import lib, solvers, synth
@@ -50,25 +53,25 @@ def measure(nao: int, naux: int, slices: int = 5, nts: int = 80, mesh=(2, 2, 2),
     try:
         G = torch.from_numpy(s.G).to(f"cuda:{device}")
         Sig = torch.empty_like(G)
-        out = {}
-        for bn in candidates:
-            ctx.set_tile_width(bn)
-            ctx.gw_sigma_device(G.data_ptr(), Sig.data_ptr())  # warm-up (buffers, maps)
-            torch.cuda.synchronize(device)
-            ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
-            ev[0].record()
-            for _ in range(reps):
+        ms = {int(bn): [] for bn in candidates}
+        for rep in range(reps + 1):  # in turn, so that clocks and neighbours weigh on all alike; the first round warms up
+            for bn in ms:
+                ctx.set_tile_width(bn)
+                torch.cuda.synchronize(device)
+                ev = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+                ev[0].record()
                 ctx.gw_sigma_device(G.data_ptr(), Sig.data_ptr())
-            ev[1].record()
-            torch.cuda.synchronize(device)
-            out[int(bn)] = ev[0].elapsed_time(ev[1]) / reps
-        return out
+                ev[1].record()
+                torch.cuda.synchronize(device)
+                if rep > 0:
+                    ms[bn].append(ev[0].elapsed_time(ev[1]))
+        return {bn: round(min(t), 1) for bn, t in ms.items()}  # (below a tenth lies the clocks' noise: a tie is no limit)
     finally:
         ctx.close()
 
 
 def tune(shapes, **kw) -> dict:
-    """{"<nao>x<naux>": {"bn": fastest width, "ms": {width: ms}}} over `shapes` [(nao, naux)]."""
+    """{"<nao>x<naux>": {"bn": fastest limit, "ms": {limit: ms}}} over `shapes` [(nao, naux)]."""
     table = {}
     for nao, naux in shapes:
         ms = measure(nao, naux, **kw)
@@ -86,7 +89,7 @@ def main(argv=None):
     import torch
     doc = {"device": torch.cuda.get_device_name(0), "slices": args.slices,
            "workload": "synthetic system per shape: 2x2x2 mesh, ntau = 80, beta = 100, one self-energy, "
-                       "CUDA events over 3 calls after a warm-up call",
+                       "fastest of 9 calls, the limits in turn (CUDA events)",
            "shapes": table}
     with open(args.out, "w") as f:
         json.dump(doc, f, indent=1)

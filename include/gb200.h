@@ -111,9 +111,10 @@ int gb200_set_q_range(gb200_context* ctx, int q_begin, int q_end);
 int gb200_gw_sigma_batch_device(gb200_context* const* ctxs, int n, const double* const* G_dev,
                                 double* const* Sigma_dev, void* stream);
 
-/* Column tile width of the split-precision contractions of a context (a multiple of 16, at most
- * the widest tile that S slices allow; 0: the widest).  The batched workload's autotuner picks it
- * per (nao, naux). */
+/* Upper limit of the column tile width of the split-precision contractions of a context (rounded
+ * down to a multiple of 16); below it, and below the widest tile that S slices allow, the library
+ * chooses the width per contraction.  0: no limit.  The results do not depend on it.  The batched
+ * workload's autotuner picks it per (nao, naux). */
 int gb200_set_tile_width(gb200_context* ctx, int bn);
 
 /* q-sharded storage of the GW integrals: only the stored pairs `pair_ids` (indices

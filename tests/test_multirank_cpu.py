@@ -181,7 +181,7 @@ def test_batch_memory_shares_are_proportional():
 
 
 def test_tile_table_lookup():
-    """The autotuner's table is read by nearest measured (nao, naux); without one the widest tile."""
+    """The autotuner's table is read by nearest measured (nao, naux); without one there is no limit."""
     from gb200 import tune
     table = {"8x32": {"bn": 32}, "40x200": {"bn": 80}, "48x288": {"bn": 96}}
     assert tune.choose_tile(9, 36, table) == 32
