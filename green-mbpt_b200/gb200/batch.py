@@ -5,9 +5,10 @@ CUDA stream.  `run_gw_grouped` evaluates all of them in one library call whose c
 are grouped persistent launches over the tiles of every system (gb200_gw_sigma_batch_device), with
 limits of the tile width from the autotuner's table (`apply_tiles`).  `run_gw` instead issues the
 self-energy of every system from a pool of host threads.  The library calls release the
-interpreter lock, so the systems' kernels are queued on different streams and
-overlap on the device wherever one system does not fill it: the slicing and FP64 kernels of one system run beside the contraction kernel of another.  Results are identical to
-running the systems one by one: every context computes exactly what it would alone.
+interpreter lock, so the systems' kernels are queued on different streams and overlap on the device
+wherever one system does not fill it: the slicing and FP64 kernels of one system run beside the
+contraction kernel of another.  Results are identical to running the systems one by one: every
+context computes exactly what it would alone.
 """
 from __future__ import annotations
 

@@ -70,12 +70,12 @@ def test_full_sigma_within_bound_on_workload_shapes(gpu):
 @pytest.mark.parametrize("name", ["small", "small_ns2"])
 def test_split_matches_cpu_model_of_its_arithmetic(gpu, name):
     """The GPU split engine against oracle/split_model.py, the CPU restatement of its arithmetic
-    (exponents per row and column with one bit of headroom, rounded balanced base-128 digits, kept
+    (exponents per row and column with one bit of headroom, rounded balanced base-256 digits, kept
     diagonals), at three slices.  On these systems all k-points form one block and no contraction
     is chunked, so both form the same exponent groups and the same exact integer digit products:
     they agree to 1e-10 relative, while both differ from the FP64 result by about 1e-6 relative and
     truncated digits would differ from balanced ones by as much.  (Three slices: the digit quantum,
-    2^-21 of the row maximum, is far above the FP64 round-off in which the two differ, so no
+    2^-23 of the row maximum, is far above the FP64 round-off in which the two differ, so no
     rounding decision of a later contraction's slicing flips between them.)"""
     import split_model as SM
     s = system(name)
@@ -88,12 +88,9 @@ def test_split_matches_cpu_model_of_its_arithmetic(gpu, name):
 
 
 @pytest.mark.parametrize("ns", [1, 2])
-def test_exponent_sinks_match_separate_exponent_passes(gpu, ns):
-    """With nao a multiple of 8 the tensor-core engine records the column exponents of Y2 (the
-    operand of (f)) in the epilogue of (e) as it stores Y2, and skips the slicer's exponent pass
-    for Y2; the validation engine still runs that pass.  No contraction is chunked here, so both
-    see the same exponents and the self-energies agree bit for bit; at 5 slices both are within
-    1e-8 of the FP64 path."""
+def test_engines_agree_at_whole_column_groups(gpu, ns):
+    """nao a multiple of 8, so that every group of 8 result columns of the epilogue is full: the two
+    engines agree bit for bit at 5 slices, one spin and two, and both are within 1e-8 of FP64."""
     from gb200 import synth
     s = synth.make_system(mesh=(2, 2, 1), nao=8, naux=24, ns=ns, beta=20.0, nts=20, eps_range=2.0, seed=5 + ns)
     a = sigma_split(s, 5, 1)

@@ -61,7 +61,8 @@ def test_balanced_digits_match_bottom_up_construction(harness):
         vals += [int(v) for v in rng.integers(-(lim - 1), lim, 200, dtype=np.int64)]
         cases += [(S, v) for v in vals]
     inp = "".join(f"{S} {v}\n" for S, v in cases)
-    out = subprocess.run([harness], input=inp, capture_output=True, text=True, check=True).stdout.split("\n")
+    out = subprocess.run([harness], input=inp, capture_output=True, text=True, check=True).stdout.splitlines()
+    assert len(out) == len(cases)
     for (S, X), line in zip(cases, out):
         got = [int(t) for t in line.split()]
         assert got == bottom_up(X, S), (S, X, got)
@@ -135,7 +136,8 @@ def test_packed_digit_words_match_single_digits(tmp_path):
             vals.append(0.0)
         cases += [(S, vals[i:i + 4]) for i in range(0, len(vals), 4)]
     inp = "".join(f"{S} " + " ".join(repr(v) for v in x) + "\n" for S, x in cases)
-    out = subprocess.run([str(exe)], input=inp, capture_output=True, text=True, check=True).stdout.split("\n")
+    out = subprocess.run([str(exe)], input=inp, capture_output=True, text=True, check=True).stdout.splitlines()
+    assert len(out) == len(cases)
     for (S, x), line in zip(cases, out):
         t = [int(v) for v in line.split()]
         assert t[:4] == [int(np.rint(v)) for v in x], (S, x, t[:4])

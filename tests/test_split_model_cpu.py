@@ -5,7 +5,7 @@ import numpy as np
 
 def test_split_model_error_falls_by_the_digit_base():
     """The CPU model of the split arithmetic (oracle/split_model.py): each added slice divides the
-    error of a product by about 2^7, and small integers are represented exactly."""
+    error of a product by about 2^8 (base-256 digits), and small integers are represented exactly."""
     import split_model as SM
     rng = np.random.default_rng(3)
     A = rng.standard_normal((24, 40)) + 1j * rng.standard_normal((24, 40))

@@ -51,8 +51,10 @@ def test_wide_digits_match_bottom_up_construction(tmp_path):
         lim = 1 << (8 * S - 2)
         vals = [0, 1, -1, 127, 128, -128, -129, 255, 256, lim, -lim, lim - 1, lim // 2] + [int(x) for x in rng.integers(-lim, lim, 200)]
         cases += [(S, v) for v in vals]
-    out = subprocess.run([str(exe)], input="\n".join(f"{S} {v}" for S, v in cases), capture_output=True, text=True).stdout
-    for (S, v), line in zip(cases, out.strip().splitlines()):
+    r = subprocess.run([str(exe)], input="\n".join(f"{S} {v}" for S, v in cases), capture_output=True, text=True)
+    lines = r.stdout.strip().splitlines()
+    assert r.returncode == 0 and len(lines) == len(cases)
+    for (S, v), line in zip(cases, lines):
         got = [int(x) for x in line.split()]
         assert got[0::2] == bottom_up(v, S) and got[1::2] == bottom_up(-v, S), (S, v)
         assert abs(got[0]) <= 64 and abs(got[1]) <= 64
