@@ -86,7 +86,10 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t phase) {
   return ok != 0;
 }
 
-// Bounded wait: returns false on timeout.
+// Bounded wait: returns false on timeout.  Warps whose lanes all touch what a barrier guards call it from every lane, and
+// vote on the outcome: each lane then has its own acquire.  (One lane polling for the others needs a __syncwarp behind it,
+// because a shuffle of the outcome orders no memory, and the loop of a single lane was slower: with it gw_split_mid took
+// 171.7 ms, iteration_split 51.0 and batch_uneven 255 instead of 160.0, 47.6 and 234.)
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
   if (mbar_try_wait(bar, phase)) return true;
   const long long t0 = clock64();
@@ -95,15 +98,6 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t phase, volatil
     if (clock64() - t0 > WAIT_LIMIT) return false;
   }
   return true;
-}
-
-// The whole warp waits, one lane polls.  The shuffle brings the other lanes the outcome but orders no memory; __syncwarp
-// is what carries the polling lane's acquire over to their reads and writes.
-__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t phase, volatile int* abort_flag) {
-  int ok = 1;
-  if (threadIdx.x % 32 == 0) ok = mbar_wait(bar, phase, abort_flag);
-  __syncwarp();
-  return __shfl_sync(0xffffffffu, ok, 0) != 0;
 }
 
 __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* map, int x, int y, int z, uint64_t* bar) {
@@ -916,7 +910,8 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
       const bool cin = lane < clim;
       const int e0 = cin ? eA[lane] : 0;
       const int64_t o0 = cin ? q.C.row(m0 + lane) : 0;
-      if (!mbar_wait_warp(&tabe_bar[set], ((tcount >> 1) & 1) ^ 1, abort_flag)) {
+      const bool ok = mbar_wait(&tabe_bar[set], ((tcount >> 1) & 1) ^ 1, abort_flag);
+      if (!__all_sync(0xffffffffu, ok)) {
         if (lane == 0) {
           atomicExch(p.err, SERR_TIMEOUT_TABLES);
           *abort_flag = 1;
@@ -982,8 +977,8 @@ __global__ void __launch_bounds__(NWARPS * 32, 1)
     int buf = 0;
     for (uint32_t t = t_first; t < t_end; t += t_step, ++tcount) {
       const int set = (int)(tcount & 1);
-      if (!mbar_wait_warp(&tabf_bar[set], (tcount >> 1) & 1, abort_flag) ||
-          !mbar_wait_warp(&accf_bar[buf], acc_ph, abort_flag)) {
+      const bool ok = mbar_wait(&tabf_bar[set], (tcount >> 1) & 1, abort_flag) && mbar_wait(&accf_bar[buf], acc_ph, abort_flag);
+      if (!__all_sync(0xffffffffu, ok)) {
         if (lane == 0) {
           atomicExch(p.err, SERR_TIMEOUT_EPILOGUE);
           *abort_flag = 1;
