@@ -38,6 +38,9 @@ struct MirrorTransforms {
   std::vector<std::complex<double>> half;  // [nts / 2][nu]: the mean of its mirrored rows
 };
 
+// |z| without the scaling by which std::abs guards the ends of the double range
+inline double modulus(std::complex<double> z) { return std::sqrt(std::norm(z)); }
+
 inline MirrorTransforms mirror_transforms(const std::complex<double>* F, const std::complex<double>* B, int nts, int nw) {
   const int nth = nts / 2;
   MirrorTransforms m;
@@ -88,68 +91,67 @@ inline MirrorTransforms mirror_transforms(const std::complex<double>* F, const s
     m.change = m.bound = asym / bmax;
     return m;
   }
-  // out += X Y for a row X [n] and Y [n][nth], and the sum of magnitudes
-  struct Acc {
-    std::vector<double> re, im, mag;
-    explicit Acc(int n) : re(n), im(n), mag(n) {}
-    void clear() {
-      std::fill(re.begin(), re.end(), 0.0);
-      std::fill(im.begin(), im.end(), 0.0);
-      std::fill(mag.begin(), mag.end(), 0.0);
-    }
-    void add(std::complex<double> x, const double* yr, const double* yi, const double* ym, int n) {
-      const double xr = x.real(), xi = x.imag(), xm = std::hypot(xr, xi);
+  // a row of nth complex sums and the sum of magnitudes (separate arrays: the loop vectorizes)
+  struct Row {
+    std::vector<double> v;
+    int n;
+    explicit Row(int n_) : v(3 * (size_t)n_), n(n_) {}
+    void clear() { std::fill(v.begin(), v.end(), 0.0); }
+    void add(std::complex<double> x, const Row& y) {  // += x y
+      const double xr = x.real(), xi = x.imag(), xm = modulus(x);
+      double* __restrict re = v.data();
+      double* __restrict im = re + n;
+      double* __restrict mag = im + n;
+      const double* __restrict yr = y.v.data();
+      const double *yi = yr + n, *ym = yi + n;
       for (int t = 0; t < n; ++t) {
         re[t] += xr * yr[t] - xi * yi[t];
         im[t] += xr * yi[t] + xi * yr[t];
         mag[t] += xm * ym[t];
       }
     }
-  };
-  auto planes = [&](const std::vector<std::complex<double>>& y) {
-    std::vector<double> p(3 * y.size());
-    for (size_t i = 0; i < y.size(); ++i) {
-      p[i] = y[i].real();
-      p[y.size() + i] = y[i].imag();
-      p[2 * y.size() + i] = std::abs(y[i]);
+    void set(int t, std::complex<double> z) {
+      v[t] = z.real();
+      v[n + t] = z.imag();
+      v[2 * (size_t)n + t] = modulus(z);
     }
-    return p;
+    std::complex<double> at(int t) const { return {v[t], v[n + t]}; }
+    double sum_of_magnitudes(int t) const { return v[2 * (size_t)n + t]; }
   };
-  std::vector<std::complex<double>> dF;  // rows that a merge moves
+  std::vector<Row> rows(nu, Row(nth)), moves;
+  for (int u = 0; u < nu; ++u)
+    for (int t = 0; t < nth; ++t) rows[u].set(t, m.fwd[(size_t)u * nth + t]);
+  // what a merge takes from its members' rows sums to zero, so one of them (the group's first) goes without: B F changes
+  // by the sum over the others of (B_member - B_first) dF_member
   std::vector<int> moved;
   for (int n = 0; n < nw; ++n) {
-    if (members[group[n]] == 1) continue;
+    if (n == first[group[n]]) continue;
     moved.push_back(n);
-    for (int t = 0; t < nth; ++t) dF.push_back(F[(size_t)n * nth + t] - m.fwd[(size_t)group[n] * nth + t]);
+    moves.emplace_back(nth);
+    for (int t = 0; t < nth; ++t) moves.back().set(t, F[(size_t)n * nth + t] - m.fwd[(size_t)group[n] * nth + t]);
   }
-  const std::vector<double> pf = planes(m.fwd), pd = planes(dF);
-  const size_t nf = m.fwd.size(), nd = dF.size();
   // the composed transform's size, and per time the change: (full - half) fwd + B dF
-  Acc s(nth), skew(nth), d(nth);
+  Row s(nth), skew(nth), d(nth);
   double scale = 0.0, change = 0.0, bound = 0.0;
   for (int t = 0; t < nth; ++t) {
     s.clear();
     skew.clear();
     for (int u = 0; u < nu; ++u) {
-      const double *yr = &pf[(size_t)u * nth], *yi = yr + nf, *ym = yi + nf;
       const std::complex<double> h = m.half[(size_t)t * nu + u];
-      s.add(h, yr, yi, ym, nth);
-      skew.add(m.full[(size_t)t * nu + u] - h, yr, yi, ym, nth);
+      s.add(h, rows[u]);
+      skew.add(m.full[(size_t)t * nu + u] - h, rows[u]);
     }
+    for (int k = 0; k < nth; ++k) scale = std::max(scale, modulus(s.at(k)));
     for (int mirror = 0; mirror < 2; ++mirror) {
-      const int row = mirror ? nts - 1 - t : t;
+      const std::complex<double>* b = B + (size_t)(mirror ? nts - 1 - t : t) * nw;
       d.clear();
-      for (size_t i = 0; i < moved.size(); ++i) {
-        const double *yr = &pd[i * nth], *yi = yr + nd, *ym = yi + nd;
-        d.add(B[(size_t)row * nw + moved[i]], yr, yi, ym, nth);
-      }
+      for (size_t i = 0; i < moved.size(); ++i) d.add(b[moved[i]] - b[first[group[moved[i]]]], moves[i]);
       const double sign = mirror ? -1.0 : 1.0;  // the mirrored row of full - half is minus this one
       for (int k = 0; k < nth; ++k) {
-        change = std::max(change, std::hypot(sign * skew.re[k] + d.re[k], sign * skew.im[k] + d.im[k]));
-        bound = std::max(bound, skew.mag[k] + d.mag[k]);
+        change = std::max(change, modulus(sign * skew.at(k) + d.at(k)));
+        bound = std::max(bound, skew.sum_of_magnitudes(k) + d.sum_of_magnitudes(k));
       }
     }
-    for (int k = 0; k < nth; ++k) scale = std::max(scale, std::hypot(s.re[k], s.im[k]));
   }
   m.change = scale > 0.0 ? change / scale : change;
   m.bound = scale > 0.0 ? bound / scale : bound;
