@@ -1302,10 +1302,10 @@ int64_t kmax_for(int S) {
 }
 
 // Tile width of a problem, in real columns of the embedded operand (2 M of them): one TMEM accumulator set of up to 512
-// columns (two of half that in overlap mode), or the context's chosen width, and below that the multiple of 16 with
-// which the tiles cost least: a K step moves the planes of 128 rows and BN columns from L2 (33 bytes a cycle and SM
-// measured), which takes longer than its MMAs; in overlap mode a tile costs its epilogue and about 16 columns' worth
-// of waits.
+// columns (two of half that in overlap mode), no more than the context's limit, and below that the multiple of 16 with
+// which the tiles cost least: their number times the rows and columns of planes that a K step brings from L2; in overlap
+// mode a tile costs its epilogue and about 16 columns' worth of waits.  Five slices at nao = 24 to 48: a limit of 80, 64,
+// 48 or 32 columns is 0-6, 0-8, 6-12 or 21-36 % slower than none (gb200/tile_table.json).
 int tile_width(const Context& c, int S, int64_t M, bool overlap) {
   int top = max_bn(S, overlap ? 256 : 512);
   if (c.tile_bn > 0) top = std::min(top, std::max(16, c.tile_bn / 16 * 16));

@@ -11,9 +11,10 @@
 //
 // Two or three CTAs of 128 threads share an SM (255 or 168 registers a thread): one of them stores its tile or fills
 // its ring while another multiplies (three instead of two for the smaller tiles: 10.0 -> 9.0 ms on the exchange below,
-// 132 -> 122 ms on a two-spin self-energy at nao = 26).  What bounds it is the FP64 tensor pipe (37 TFLOP/s from registers): 71 % of it
-// on 150 x 150 x 10816, half on contractions as short as K = 26, where the index maps and the stores count.  Copies
-// issued between the products instead of before them were slower (their address loads stall the warp that multiplies).
+// 132 -> 122 ms on a two-spin self-energy at nao = 26).  What bounds it is the FP64 tensor pipe (37 TFLOP/s from
+// registers): 76 % of its cycles on 250 x 250 x 3200 and 250 x 1600 x 250, 54 to 62 % where K = 40, where the ring's fill,
+// the index maps and the stores count.  Copies issued between the products instead of before them were slower (their
+// address loads stall the warp that multiplies).
 // Exchange of a Fock build at nk = 27, nao = 40, NQ = 250: 29.4 -> 9.0 ms against the 64 x 64 kernel with register
 // staging that this one replaced.
 // Contractions with few tiles split K over a cluster of up to 8 CTAs and sum the parts through distributed
@@ -270,10 +271,12 @@ struct Variant {
   int tm, tn, wn;
 };
 
-// Time of a variant in SM cycles.  Per K step of one element a CTA needs MT NTL 4 / 65 cycles of the FP64 tensor
-// pipe (65 multiply-adds a cycle and SM: 37 TFLOP/s measured from registers) and (MT + NTL) 16 bytes from L2 at
-// about 19 bytes a cycle and SM; ~900 cycles a tile are the ring's fill and the stores that the other CTA of the
-// SM does not hide.  Tiles are spread over 148 SMs.
+// Time of a variant in SM cycles, up to what all variants share.  Per K step of one element a CTA needs MT NTL 4 / 65
+// cycles of the FP64 tensor pipe (65 multiply-adds a cycle and SM: 37 TFLOP/s measured from registers) and (MT + NTL) 16
+// bytes from L2 at 19 bytes a cycle and SM; 900 cycles a tile are the ring's fill and the stores that the other CTA of the
+// SM does not hide.  The last two are not rates of the hardware but the values at which the variants rank as they measure:
+// with 12 bytes gw at nao = 26, ns = 2 takes 128.5 ms instead of 122.1, with 33 the adjoint at nao = 20 takes 127.5
+// instead of 114.1, and 120.4 with 500 cycles, 115.3 with 1500; Fock builds do not care.  Tiles are spread over 148 SMs.
 double variant_cost(const Variant& v, int64_t M, int64_t N, int64_t K, int64_t nbatch, int ks) {
   const double mt = 8.0 * v.tm, nt = 8.0 * v.tn * v.wn;
   const double tiles = std::ceil(M / mt) * std::ceil(N / nt) * (double)nbatch * ks;
