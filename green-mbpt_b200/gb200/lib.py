@@ -215,7 +215,7 @@ class Context:
         self._check(self._L.gb200_set_contraction_slices(self._h, arr))
 
     def set_memory_budget(self, nbytes: float):
-        """Bytes the blocked intermediates of one call may use (0: a share of the free memory)."""
+        """Bytes the blocked intermediates of one call, slice planes included, may use (0: a share of the free memory)."""
         self._check(self._L.gb200_set_memory_budget(self._h, float(nbytes)))
 
     def set_split_engine(self, engine: int):

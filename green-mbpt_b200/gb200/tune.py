@@ -54,7 +54,7 @@ def measure(nao: int, naux: int, slices: int = 5, nts: int = 80, mesh=(2, 2, 2),
         G = torch.from_numpy(s.G).to(f"cuda:{device}")
         Sig = torch.empty_like(G)
         ms = {int(bn): [] for bn in candidates}
-        for rep in range(reps + 1):  # in turn, so that clocks and neighbours weigh on all alike; the first round warms up
+        for rep in range(reps + 1):  # in turn, so that the clocks weigh on all alike; the first turn warms up
             for bn in ms:
                 ctx.set_tile_width(bn)
                 torch.cuda.synchronize(device)
